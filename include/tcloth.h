@@ -512,11 +512,12 @@ tc_status tc_mesh_topology(tc_mesh *m, uint32_t *adj_off, uint32_t *adj_idx, uin
 tc_status tc_set_profiling_enabled(tc_sim *s, int enable);
 tc_status tc_take_profile(tc_sim *s, char *names, size_t names_len, float *ms, uint32_t *launches,
                           uint32_t max_entries, uint32_t *n_entries);
-/* Persistent solver (default on when the device supports cooperative
- * launch): the constraint phase of a substep (of a whole frame when
+/* Persistent solver, a launch shape the caller can choose: the constraint phase of a substep (of a whole frame when
  * self-collision is off) is one cooperative launch whose colours are
  * separated by bounded grid barriers; off = one launch per colour.  Both give
- * the same bits.  A barrier that waits past its poll limit makes tc_step
+ * the same bits.  Without a choice the library picks: the resident solver
+ * (one thread-block cluster with the cloth on chip) where the cloth fits it,
+ * else one launch per colour, and for batched instances the persistent one.  A barrier that waits past its poll limit makes tc_step
  * return TC_ERR_TIMEOUT.  New; the reference dispatches one pass per colour
  * (dispatch.rs:1449-1455). */
 tc_status tc_set_persistent_solver(tc_sim *s, int enable);
@@ -528,7 +529,8 @@ tc_status tc_set_persistent_solver(tc_sim *s, int enable);
  * bin's vertex records held in the cluster's shared memory for the whole
  * frame, split into one slice per CTA and reached across CTAs through
  * distributed shared memory; needs every instance within 8 x the per-CTA
- * capacity).  TC_ERR_INVALID when a mode is not applicable.  Used by the
+ * capacity); 4 the library's choice (the default: see
+ * tc_set_persistent_solver).  TC_ERR_INVALID when a mode is not applicable.  Used by the
  * autotuner.  Results do not change. */
 tc_status tc_set_launch_config(tc_sim *s, int persistent, uint32_t blocks_per_sm);
 tc_status tc_get_launch_limits(tc_sim *s, uint32_t *max_blocks_per_sm, uint32_t *num_sms);

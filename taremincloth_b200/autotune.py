@@ -1,6 +1,8 @@
 """Autotuner for a simulator's launch shape and, on request, its hash cell.
 
 Launch shape (results never change, only speed):
+* the library's own choice (the resident solver where the cloth fits one
+  thread-block cluster),
 * the launch-per-colour path at each tile size (threads per block of the
   per-colour constraint launches: 128, 256, 512),
 * the persistent solver at every blocks-per-SM value the occupancy allows,
@@ -73,7 +75,8 @@ def autotune(sim, dt, substeps, frames=3, verbose=False, tune_cell_sizes=None):
     x, _, v = sim.get_state()
     x, v = x.copy(), v.copy()
     max_per_sm, _ = sim.get_launch_limits()
-    trials = [(False, 0, b) for b in (128, 256, 512)]
+    trials = [(4, 0, 256)]
+    trials += [(False, 0, b) for b in (128, 256, 512)]
     trials += [(True, b, 256) for b in range(1, min(max_per_sm, 4) + 1)]
     for mode in (2, 3):  # cluster solver, staged cluster solver
         try:

@@ -32,6 +32,7 @@
 #include "paircache_kernels.cuh"
 #include "collider_prep.cuh"
 #include "solver_kernels.cuh"
+#include "resident_solver.cuh"
 #include "warmstart.cuh"
 
 namespace tcloth {
@@ -738,6 +739,18 @@ struct Sim {
   DBuf<uint4> st_bids;
   DBuf<float4> st_dpar, st_bpar;
   DBuf<float> st_dlam, st_blam;
+  // resident solver (resident_solver.cuh): one cluster of rs_ctas CTAs with
+  // the cloth's vertices on chip; 0 = the cloth does not fit or the device
+  // cannot.  The tables follow from the mesh; pins and compliances are
+  // refreshed when they change.
+  uint32_t rs_ctas = 0, rs_chunk = 0, rs_ccap = 0, rs_nsteps = 0, rs_ndsteps = 0;
+  bool rs_full = false, rs_built = false, rs_par_stale = true, rs_pins_stale = true;
+  size_t rs_smem = 0;
+  std::vector<uint32_t> col_order_h, rs_sid_h;  // Morton order of the initial positions; slice and slot of a vertex
+  DBuf<uint32_t> rs_sid, rs_tab, rs_perm, rs_pin_tab, rs_pin_idx, rs_sew_tab, rs_sew_idx;
+  DBuf<uint2> rs_ids, rs_gate_ids;
+  DBuf<float4> rs_par;
+  DBuf<float> rs_gate_gap;
   std::vector<uint2> inst_prims_h;
   DBuf<uint32_t> vinst;
   DBuf<uint2> inst_prims;
@@ -747,6 +760,8 @@ struct Sim {
   DBuf<float4> pin_t;
   // persistent solver (one cooperative launch per substep / frame)
   bool persistent = true;
+  // launch shape not chosen by the caller: see use_resident() / use_persistent()
+  bool launch_auto = true;
   unsigned int persist_blocks = 0, persist_max_per_sm = 0, num_sms = 0, persist_bone_per_sm = 0;
   unsigned int spin_limit = 1u << 22;  // ~0.5 s of polling per barrier
   DBuf<GridBar> bar;
@@ -993,6 +1008,7 @@ struct Sim {
     dist_ids.upload(ids, st);
     dist_par.upload(par, st);
     st_stale = true;  // the staged solver's copies follow on its next frame
+    rs_par_stale = true;
     TC_CK(cudaStreamSynchronize(st));
   }
   void upload_bend() {
@@ -1005,6 +1021,7 @@ struct Sim {
     }
     bend_ids.upload(ids, st);
     st_stale = true;
+    rs_par_stale = true;
     bend_par.upload(par, st);
     TC_CK(cudaStreamSynchronize(st));
   }
@@ -1035,6 +1052,7 @@ struct Sim {
       std::vector<uint32_t> ord(n);
       for (uint32_t i = 0; i < n; ++i) ord[i] = code[i].second;
       col_order.upload(ord, st);
+      col_order_h = std::move(ord);
     }
     nd = uint32_t(m.dist.size());
     nb = uint32_t(m.bend.size());
@@ -1179,6 +1197,7 @@ struct Sim {
         st_max_active = ncl;
       }
       num_sms = unsigned(nsm);
+      plan_resident();
       if (!persist_blocks) persistent = false;
     }
     pin_v.alloc(1); pin_t.alloc(1);
@@ -1262,6 +1281,7 @@ struct Sim {
   void upload_pins() {
     cl_stale = true;
     st_stale = true;
+    rs_pins_stale = true;
     std::vector<uint32_t> v;
     std::vector<float4> t;
     for (const auto& kv : pins) {
@@ -1825,6 +1845,192 @@ struct Sim {
     if (a.ca.bone.nbones > 0) TC_CK(cudaLaunchKernelEx(&cfg, k_solver_staged<kStageCtas, true>, a, t));
     else TC_CK(cudaLaunchKernelEx(&cfg, k_solver_staged<kStageCtas, false>, a, t));
   }
+  using ResidentKernel = void (*)(SolverArgs, ResidentArgs);
+  static ResidentKernel resident_kernel(bool full, bool with_bone) {
+    if (full) return with_bone ? k_solver_resident<true, true> : k_solver_resident<true, false>;
+    return with_bone ? k_solver_resident<false, true> : k_solver_resident<false, false>;
+  }
+  void resident_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, uint32_t ctas, size_t smem) {
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(tcloth::kResThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ctas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+  }
+  // Size of the cluster for this cloth (rs_ctas = 0: not resident).
+  void plan_resident() {
+    rs_ctas = 0;
+    if (n == 0 || nd + nb == 0) return;
+    int optin = 0;
+    TC_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    rs_nsteps = rs_ndsteps = 0;
+    for (uint32_t c : m.dist_cnt) rs_nsteps += c ? 1u : 0u;
+    rs_ndsteps = rs_nsteps;
+    for (uint32_t c : m.bend_cnt) rs_nsteps += c ? 1u : 0u;
+    uint32_t k = 1;
+    // about 512 vertices per CTA: one constraint per thread in a colour step.
+    // Fewer per CTA buys nothing (8,065 vertices: 0.89 ms a frame of 750 steps
+    // at 256 and 512, 0.97 at 1,024; 265 vertices: 0.20 on one CTA, 0.29 on two)
+    while (k < tcloth::kResMaxCtas && (n + k - 1) / k > 512u) k *= 2;
+    // constraints owned per CTA
+    const uint32_t chunk = (n + k - 1) / k;
+    if (chunk > 65535u) return;
+    std::vector<uint32_t> pos(n), own(k, 0u);
+    for (uint32_t q = 0; q < n; ++q) pos[col_order_h[q]] = q;
+    for (const auto& c : dist_h) ++own[pos[c.v0] / chunk];
+    for (const auto& c : bend_h) ++own[pos[c.v2] / chunk];
+    const uint32_t ccap = (*std::max_element(own.begin(), own.end()) + 1u) & ~1u;
+    const size_t recs = size_t(ccap) * 24u + (size_t(rs_nsteps) + 1u) * 4u;
+    const bool full = size_t(chunk) * 48u + recs <= size_t(optin);
+    const size_t smem = size_t(chunk) * (full ? 48u : 16u) + recs;
+    if (smem > size_t(optin)) return;
+    for (bool with_bone : {false, true}) {
+      const void* f = reinterpret_cast<const void*>(resident_kernel(full, with_bone));
+      int ncl = 0;
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[1];
+      resident_config(cfg, attr, k, smem);
+      if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess ||
+          cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&ncl, f, &cfg) != cudaSuccess || ncl < 1) {
+        cudaGetLastError();
+        return;
+      }
+    }
+    rs_ctas = k; rs_chunk = chunk; rs_ccap = ccap; rs_full = full; rs_smem = smem;
+  }
+  // Tables of the resident solver: every colour's constraints ordered by the
+  // slice position of their first projected vertex, so that the owner's
+  // constraints are contiguous and neighbouring lanes read neighbouring slots.
+  void ensure_resident() {
+    if (!use_resident()) return;
+    const uint32_t K = rs_ctas;
+    if (!rs_built) {
+      std::vector<uint32_t> sid(n), pos(n);
+      for (uint32_t q = 0; q < n; ++q) {
+        const uint32_t v = col_order_h[q];
+        pos[v] = q;
+        sid[v] = ((q / rs_chunk) << 16) | (q % rs_chunk);
+      }
+      // records by (slice, step, slice position of the first vertex): bucket
+      // by position, then walk each slice's buckets; bending constraints
+      // carry the top bit
+      const uint32_t ndc = uint32_t(m.dist_cnt.size()), nbc = uint32_t(m.bend_cnt.size());
+      auto each = [&](auto&& f) {
+        uint32_t step = 0;
+        for (uint32_t c = 0; c < ndc; ++c) {
+          for (uint32_t k = m.dist_off[c]; k < m.dist_off[c] + m.dist_cnt[c]; ++k) f(k, dist_h[k].v0, step);
+          step += m.dist_cnt[c] ? 1u : 0u;
+        }
+        for (uint32_t c = 0; c < nbc; ++c) {
+          for (uint32_t k = m.bend_off[c]; k < m.bend_off[c] + m.bend_cnt[c]; ++k) f(k | 0x80000000u, bend_h[k].v2, step);
+          step += m.bend_cnt[c] ? 1u : 0u;
+        }
+      };
+      const uint32_t total = nd + nb, S1 = rs_nsteps + 1;
+      std::vector<uint32_t> off(size_t(n) + 1, 0u), list(total), step_at(total), tab(size_t(K) * S1 + 1, 0u);
+      each([&](uint32_t, uint32_t v, uint32_t step) {
+        ++off[pos[v] + 1];
+        ++tab[size_t(pos[v] / rs_chunk) * S1 + step + 1];  // (the slot after a slice's last step stays 0)
+      });
+      for (uint32_t q = 0; q < n; ++q) off[q + 1] += off[q];
+      // a slice's end is the next slice's begin
+      for (size_t q = 1; q < tab.size(); ++q) tab[q] += tab[q - 1];
+      std::vector<uint32_t> fill(off.begin(), off.end() - 1), head(tab), perm(total);
+      each([&](uint32_t k, uint32_t v, uint32_t step) {
+        const uint32_t at = fill[pos[v]]++;
+        list[at] = k;
+        step_at[at] = step;
+      });
+      for (uint32_t q = 0; q < n; ++q)
+        for (uint32_t e = off[q]; e < off[q + 1]; ++e) perm[head[size_t(q / rs_chunk) * S1 + step_at[e]]++] = list[e];
+      tab.pop_back();
+      bool gated = false;
+      for (const auto& c : bend_h) gated = gated || (c.pad0 > 0.5f && c.pad0 < 1.5f);
+      std::vector<uint2> ids(total), gate(gated ? total : 0u, make_uint2(0u, 0u));
+      std::vector<float> gap(gate.size(), 0.f);
+      for (uint32_t q = 0; q < total; ++q) {
+        const uint32_t k = perm[q] & 0x7FFFFFFFu;
+        if (perm[q] >> 31) {
+          const BendC& c = bend_h[k];
+          const bool gt = c.pad0 > 0.5f && c.pad0 < 1.5f;
+          ids[q] = make_uint2((gt ? 3u : 2u) << 16 | (sid[c.v2] & 0xFFFFu), sid[c.v3]);
+          if (gt) {
+            gate[q] = make_uint2(sid[c.v0], sid[c.v1]);
+            gap[q] = c.pad1;
+          }
+        } else {
+          const DistC& c = dist_h[k];
+          ids[q] = make_uint2((c.type == 1 ? 1u : 0u) << 16 | (sid[c.v0] & 0xFFFFu), sid[c.v1]);
+        }
+      }
+      std::vector<uint32_t> stab(m.sew_cnt.size() * (K + 1)), sidx;
+      for (size_t c = 0; c < m.sew_cnt.size(); ++c)
+        for (uint32_t r = 0; r <= K; ++r) {
+          stab[c * (K + 1) + r] = uint32_t(sidx.size());
+          for (uint32_t k = m.sew_off[c]; r < K && k < m.sew_off[c] + m.sew_cnt[c]; ++k)
+            if (sid[sew_h[k].v0] >> 16 == r) sidx.push_back(k);
+        }
+      rs_sid.upload(sid, st);
+      rs_sid_h = sid;
+      rs_tab.upload(tab, st);
+      rs_perm.upload(perm, st);
+      rs_ids.upload(ids, st);
+      rs_gate_ids.upload(gate, st);
+      rs_gate_gap.upload(gap, st);
+      rs_sew_tab.upload(stab, st);
+      rs_sew_idx.upload(sidx, st);
+      rs_par.alloc(total);
+      TC_CK(cudaStreamSynchronize(st));
+      rs_built = true;
+      rs_par_stale = true;
+    }
+    if (rs_par_stale) {
+      tcloth::k_resident_gather<<<grid(nd + nb, 256), 256, 0, st>>>(nd + nb, rs_perm.p, dist_par.p, bend_par.p, rs_par.p);
+      TC_CK(cudaGetLastError());
+      rs_par_stale = false;
+    }
+    if (rs_pins_stale) {
+      std::vector<uint32_t> tab(K + 1), idx;
+      for (uint32_t r = 0; r <= K; ++r) {
+        tab[r] = uint32_t(idx.size());
+        uint32_t k = 0;
+        for (const auto& kv : pins) {  // the order of pin_v
+          if (r < K && rs_sid_h[kv.first] >> 16 == r) idx.push_back(k);
+          ++k;
+        }
+      }
+      rs_pin_tab.upload(tab, st);
+      rs_pin_idx.upload(idx, st);
+      TC_CK(cudaStreamSynchronize(st));
+      rs_pins_stale = false;
+    }
+  }
+  void launch_resident(const SolverArgs& a) {
+    const ResidentArgs t{rs_ctas, rs_chunk, rs_ccap, col_order.p, rs_sid.p, rs_nsteps, rs_ndsteps, rs_tab.p,
+                         rs_ids.p, rs_par.p, rs_gate_ids.p, rs_gate_gap.p, rs_pin_tab.p, rs_pin_idx.p,
+                         rs_sew_tab.p, rs_sew_idx.p};
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    resident_config(cfg, attr, rs_ctas, rs_smem);
+    TC_CK(cudaLaunchKernelEx(&cfg, resident_kernel(rs_full, a.ca.bone.nbones > 0), a, t));
+  }
+  // The launch shape when the caller has not chosen one.  On chip where the
+  // cloth fits one cluster: a colour step costs 0.5 to 1.1 us there.  A larger
+  // single cloth runs one launch per colour, 2.1 us a step with programmatic
+  // launches.  The cooperative kernel's grid barrier costs 5.5 us a step, so
+  // it is left to batches (one launch per frame) and to callers that ask for it.
+  bool use_resident() const { return launch_auto && rs_ctas > 0; }
+  bool use_persistent() const { return persistent && can_persist() && !(launch_auto && inst_vert_off.empty()); }
+  void launch_solver(const SolverArgs& a) {
+    if (use_resident()) launch_resident(a);
+    else launch_persistent(a);
+  }
   // the persistent path is available: cooperative launch, and with bone
   // colliders the bone instantiation fits on an SM
   bool can_persist() const { return persist_blocks > 0 && (!bone.enabled || persist_bone_per_sm > 0); }
@@ -1905,12 +2111,12 @@ struct Sim {
     const uint32_t itn = run_iters();
     const uint32_t kk = std::min(ws.k, itn > 1 ? itn - 1 : 0u);
     const WsFeatArgs fa = ws_feat_args(sp, nullptr);
-    const bool colors = !persistent || cluster_mode;
+    const bool colors = !use_persistent() || cluster_mode;
     for (uint32_t s = 0; s < substeps; ++s) {
       if (colors) {
         encode_substep_ws_colors(sp, use_coupled, itn, kk, fa);
       } else {
-        timed("predict", [&] { k_predict<<<grid(n, 256), 256, 0, st>>>(n, x4.p, p4.p, v4.p, sp); });
+        timed("predict", [&] { k_predict<<<grid(n, 256), 256, 0, st>>>(n, x4.p, p4.p, v4.p, sp, nullptr, 0u, nullptr, 0u); });
         SolverArgs a = solver_args(sp, 1, use_coupled, !(self_collision || edge_active()));
         timed("ws_check", [&] { encode_ws_res_pred(sp.dt, a.ca.bone.nbones > 0); });
         timed("ws_mlp", [&] { ws.net.infer(nullptr, &fa, ws.ppred.p, nullptr, x4.p, p4.p, local_len.p); });
@@ -1974,10 +2180,8 @@ struct Sim {
     const uint32_t npins = uint32_t(pins.size());
     const ColliderArgs ca = collider_args();
     const bool bone_col = ca.bone.nbones > 0;
-    if (nd) TC_CK(cudaMemsetAsync(dlam.p, 0, nd * sizeof(float), st));
-    if (nb) TC_CK(cudaMemsetAsync(blam.p, 0, nb * sizeof(float), st));
     if (nsw) timed("sew_shrink", [&] { launch_sew_start(dts); });
-    timed("predict", [&] { launch_k(k_predict, grid(n, 256), 256, n, x4.p, p4.p, v4.p, sp); });
+    timed("predict", [&] { launch_predict(sp); });
     timed("ws_check", [&] { encode_ws_res_pred(dts, bone_col); });
     timed("ws_mlp", [&] { ws.net.infer(nullptr, &fa, ws.ppred.p, nullptr, x4.p, p4.p, local_len.p); });
     auto iteration = [&](const unsigned int* gate) {
@@ -2088,6 +2292,9 @@ struct Sim {
     cfg.numAttrs = 1;
     TC_CK(cudaLaunchKernelEx(&cfg, kern, args...));
   }
+  void launch_predict(const SubstepParams& sp) {
+    launch_k(k_predict, grid(n, 256), 256, n, (const float4*)x4.p, p4.p, v4.p, sp, dlam.p, nd, blam.p, nb);
+  }
   void launch_collision(const ColliderArgs& ca, float dts) {
     if (ca.bone.nbones > 0) launch_k(k_collision<true>, grid(n, 128), 128, n, x4.p, p4.p, ca, dts, col_order.p);
     else launch_k(k_collision<false>, grid(n, 128), 128, n, x4.p, p4.p, ca, dts, col_order.p);
@@ -2111,20 +2318,20 @@ struct Sim {
       TC_CK(cudaGetLastError());
       return;
     }
-    if (persistent && can_persist() && !profiling && !track_residual && !ws_recording()) {
+    if ((use_resident() || use_persistent()) && !profiling && !track_residual && !ws_recording()) {
       const SubstepParams sp = make_sp(dt / float(substeps));
       if (!self_collision && !edge_active()) {
-        launch_persistent(solver_args(sp, substeps, use_coupled, true));
+        launch_solver(solver_args(sp, substeps, use_coupled, true));
       } else {
         for (uint32_t s = 0; s < substeps; ++s) {
-          launch_persistent(solver_args(sp, 1, use_coupled, false));
+          launch_solver(solver_args(sp, 1, use_coupled, false));
           if (edge_active()) encode_edge_collision();
           if (sc_due(s, substeps)) encode_self_collision(ee_due(s, substeps), s, substeps, dt);
           launch_sewing(sp.dt);  // final sewing (dispatch.rs:323-337)
           k_update_vel<<<grid(n, 256), 256, 0, st>>>(n, x4.p, p4.p, v4.p, sp.dt);
         }
       }
-      TC_CK(cudaMemcpyAsync(h_err, &bar.p->err, sizeof(int), cudaMemcpyDeviceToHost, st));
+      if (!use_resident()) TC_CK(cudaMemcpyAsync(h_err, &bar.p->err, sizeof(int), cudaMemcpyDeviceToHost, st));
       TC_CK(cudaGetLastError());
       return;
     }
@@ -2136,10 +2343,8 @@ struct Sim {
     const uint32_t npins = uint32_t(pins.size());
     ColliderArgs ca = collider_args();
     for (uint32_t s = 0; s < substeps; ++s) {
-      if (nd) TC_CK(cudaMemsetAsync(dlam.p, 0, nd * sizeof(float), st));
-      if (nb) TC_CK(cudaMemsetAsync(blam.p, 0, nb * sizeof(float), st));
       if (nsw) timed("sew_shrink", [&] { launch_sew_start(dts); });
-      timed("predict", [&] { launch_k(k_predict, grid(n, 256), 256, n, x4.p, p4.p, v4.p, sp); });
+      timed("predict", [&] { launch_predict(sp); });
       if (track_residual && s + 1 == substeps && nd + nb)
         k_residual_pred<<<grid(nd + nb, 256), 256, 0, st>>>(nd, nb, dist_ids.p, dist_par.p, bend_ids.p, bend_par.p,
                                                            p4.p, fmaxf(dts, 1e-8f),
@@ -2204,6 +2409,7 @@ struct Sim {
     if (cluster_mode && can_cluster() && cl_stale) build_cluster_tables();  // before any capture
     if (stage_mode && can_stage() && st_stale) build_stage_tables();        // before any capture
     if (edge_active()) ensure_collider_edges();                             // before any capture
+    ensure_resident();                                                      // before any capture
     // the frame's device time (last_frame_ms) includes the dynamic bone SDF rebake
     TC_CK(cudaEventRecord(ev0, st));
     dynamic_bone_update();
@@ -3569,6 +3775,13 @@ tc_status tc_set_launch_config(tc_sim* s, int persistent, uint32_t blocks_per_sm
       return;
     }
     m.stage_mode = false;
+    if (persistent == 4) {  // the default rule
+      m.cluster_mode = false;
+      m.persistent = m.persist_blocks > 0;
+      m.launch_auto = true;
+      m.mark();
+      return;
+    }
     if (persistent) {
       need(m.persist_max_per_sm > 0, "cooperative launch is not available on this device");
       need(blocks_per_sm >= 1 && blocks_per_sm <= m.persist_max_per_sm, "blocks_per_sm out of the occupancy range");
@@ -3576,6 +3789,7 @@ tc_status tc_set_launch_config(tc_sim* s, int persistent, uint32_t blocks_per_sm
     }
     m.cluster_mode = false;
     m.persistent = persistent != 0;
+    m.launch_auto = false;
     m.mark();
   });
 }
@@ -3592,6 +3806,7 @@ tc_status tc_set_persistent_solver(tc_sim* s, int enable) {
     Sim& m = S(s);
     if (enable && !m.persist_blocks) throw TcError(TC_ERR_CUDA, "cooperative launch is not available on this device");
     m.persistent = enable != 0;
+    m.launch_auto = false;
     m.mark();
   });
 }

@@ -966,8 +966,8 @@ class ClothSimulator:
         """persistent: False = one launch per colour, True = persistent cooperative
         solver with `blocks_per_sm`, 2 = cluster solver (batched instances),
         3 = staged cluster solver (batched instances, vertex records in the
-        clusters' shared memory)."""
-        mode = int(persistent) if persistent in (2, 3) and persistent is not True else int(bool(persistent))
+        clusters' shared memory), 4 = the library's choice (the default)."""
+        mode = int(persistent) if persistent in (2, 3, 4) and persistent is not True else int(bool(persistent))
         self._c(self._L.tc_set_launch_config(self._h, mode, int(blocks_per_sm)))
 
     def get_launch_limits(self):
