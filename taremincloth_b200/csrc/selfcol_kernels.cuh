@@ -50,6 +50,16 @@ struct SCArgs {
   // per vertex j: bounding box of p over j and its star triangles' vertices,
   // and the range of their motion p - x: (lo, mlo.x), (hi, mlo.y), (mhi, mlo.z)
   const float4* sbox;
+  // per star entry (j; v0, v1), aligned with star_idx: the triangle's box over
+  // p and its mean motion as seen from j: (min, motion.x), (max, motion.y),
+  // motion.z
+  const float4* st_lo;
+  const float4* st_hi;
+  const float* st_mz;
+  // vertices (edges) in Morton order of their initial positions (midpoints):
+  // the order in which k_sc_solve (k_ee) works them
+  const uint32_t* order;
+  const uint32_t* eorder;
   const int4* vcell;    // floor(p / cell) per vertex
   const float* mlen;    // |p - x| per vertex
   const int4* ecell;    // floor(midpoint / cell) per edge
@@ -114,17 +124,6 @@ __device__ __forceinline__ bool th_find(const TwoHop& t, uint32_t b, uint32_t& p
   }
   return false;
 }
-__device__ __forceinline__ bool within2_t(const TwoHop& t, uint32_t a, uint32_t b) {
-  uint32_t q;
-  if (a == b) return true;
-  return th_find(t, b, q);
-}
-__device__ __forceinline__ bool near_folded_t(const TwoHop& t, uint32_t a, uint32_t b, float d) {
-  uint32_t q;
-  if (a == b) return true;
-  if (!th_find(t, b, q)) return false;
-  return !(d < t.rest[q] * 0.5f);
-}
 __device__ __forceinline__ bool near_folded_sq_t(const TwoHop& t, uint32_t a, uint32_t b, float d2) {
   uint32_t q;
   if (a == b) return true;
@@ -159,14 +158,15 @@ __device__ __forceinline__ TwoHop stage_two_hop(const uint32_t* th_off, const ui
 
 __device__ __forceinline__ uint32_t layer_of(const float4* v4, uint32_t i) { return __float_as_uint(v4[i].w); }
 
-// Star boxes for the vertex-triangle pass (see SCArgs::sbox): one thread per
-// vertex over its star pairs.
+// Star boxes and star-entry records for the vertex-triangle pass (see
+// SCArgs::sbox, st_lo): one thread per vertex over its star pairs.
 __global__ void k_star_box(uint32_t n, const uint32_t* __restrict__ star_off, const uint2* __restrict__ star_idx,
-                           const float4* __restrict__ x4, const float4* __restrict__ p4, float4* __restrict__ sbox) {
+                           const float4* __restrict__ x4, const float4* __restrict__ p4, float4* __restrict__ sbox,
+                           float4* __restrict__ st_lo, float4* __restrict__ st_hi, float* __restrict__ st_mz) {
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
-  const V3 pj = mk(p4[j]);
-  V3 lo = pj, hi = pj, mlo = pj - mk(x4[j]), mhi = mlo;
+  const V3 pj = mk(p4[j]), pjo = mk(x4[j]);
+  V3 lo = pj, hi = pj, mlo = pj - pjo, mhi = mlo;
   for (uint32_t k = star_off[j]; k < star_off[j + 1]; ++k) {
     const uint2 pr = star_idx[k];
     const V3 a = mk(p4[pr.x]), b = mk(p4[pr.y]);
@@ -175,6 +175,11 @@ __global__ void k_star_box(uint32_t n, const uint32_t* __restrict__ star_off, co
     hi = vmax(hi, vmax(a, b));
     mlo = vmin(mlo, vmin(ma, mb));
     mhi = vmax(mhi, vmax(ma, mb));
+    const V3 tmin = vmin(vmin(pj, a), b), tmax = vmax(vmax(pj, a), b);
+    const V3 tmove = (((pj - pjo) + ma) + mb) / 3.0f;
+    st_lo[k] = make_float4(tmin.x, tmin.y, tmin.z, tmove.x);
+    st_hi[k] = make_float4(tmax.x, tmax.y, tmax.z, tmove.y);
+    st_mz[k] = tmove.z;
   }
   sbox[3 * size_t(j)] = make_float4(lo.x, lo.y, lo.z, mlo.x);
   sbox[3 * size_t(j) + 1] = make_float4(hi.x, hi.y, hi.z, mlo.y);
@@ -481,234 +486,401 @@ __device__ __forceinline__ bool near_folded_sq(const SCArgs& s, uint32_t a, uint
 }
 
 // ---------------- sc_solve: shaders/self_collision.wgsl:317-681
-// One warp per vertex i.  The 27 neighbour buckets are flattened in the
-// reference's visiting order (cx outer, cz inner, bucket order inside a cell)
-// and lane L takes flattened candidates L, L+32, ...  Contacts accumulate with
-// integer atomics (order-free); the multi-layer untangle candidate, which the
-// reference picks with a first-strict-minimum scan, is the warp argmin of
-// (distance^2, flattened position).
+// A warp works a cluster of kScV vertices that are neighbours in space.  Their
+// 27-cell neighbourhoods overlap, so the union of the buckets is scanned once:
+// the candidates are staged in shared memory, 32 / kScV of them are tested
+// against all the vertices at a time, a shared load and a dozen operations for
+// 32 pairs.  The (vertex, candidate) pairs that may matter go
+// through four more phases, each on full batches of 32 fed through queues in
+// shared memory (per vertex on config 2, 131,072 vertices):
+//   1 scan     distance against conservative reaches     (about 230 candidates
+//              a cluster)
+//   2 gate     exact bounds, two-hop exclusion, star box (48 pairs)
+//   3 box      swept box against each star triangle      (160)
+//   4 owner    ownership, two-hop exclusion              (70)
+//   5 contact  the contact math                          (20; vertex-vertex
+//              contacts, 1.5, and untangle candidates likewise)
+// One loop picks the furthest phase whose queue holds a full batch, so that
+// each phase's code exists once: inlined wherever a queue fills, the contact
+// math outgrows the instruction cache (1.25 against 0.99 ms).  Contacts
+// accumulate with integer atomics and every other outcome is independent of
+// order too; the untangle candidate, which the reference picks with a
+// first-strict-minimum scan in its visiting order (cx outer, cz inner, bucket
+// order inside a cell), is the minimum of (distance^2, that order).
+//
+// A warp per vertex (candidates over the lanes) spent 6,500 warp instructions
+// a vertex, most of them on bucket walks, compaction and batches of a few
+// lanes: 1.20 ms per pass on config 2.
 struct VertCtx {
   uint32_t index;
-  float wi;
   bool pin_i;
   V3 xi, pi;
   float mli, thi, lli;
   I3 cell;
-  uint32_t li;
-  bool untangle, track;
 };
-
-// Cheap tests of one candidate (shaders/self_collision.wgsl:356-391): bucket
-// cell match, untangle-candidate tracking, and the geometric bound; true when
-// the contact work must run.
-__device__ __forceinline__ bool sc_filter(const SCArgs& s, const VertCtx& c, const TwoHop& th, uint32_t slot,
-                                          int32_t cx, int32_t cy, int32_t cz, uint32_t t, float& best_in,
-                                          uint32_t& best_j, uint32_t& best_t) {
-  const uint32_t index = c.index;
-  // one level of loads: the three hash-ordered records of this slot
-  const int4 jc = s.vs_c[slot];
-  const float4 pj4 = s.vs_p[slot];
-  const float4 q = s.vs_q[slot];
-  const uint32_t j = (uint32_t)jc.w;
-  if (j >= s.n || j == index) return false;
-  const V3 pi = c.pi;
-  const float thi = c.thi, lli = c.lli;
-  const uint32_t li = c.li;
-  const bool track = c.track;
-  const V3 pj = mk(pj4);
-  if (!(jc.x == cx && jc.y == cy && jc.z == cz)) return false;
-  const V3 dvv = pi - pj;
-  const float d2 = dot(dvv, dvv);
-  const float thj = pj4.w, llj = q.x;
-  const float eth = fmaxf(thi + thj, fminf(lli, llj) * 0.06f);
-  const float mgd = eth + (lli + llj) * 1.3f;
-  const uint32_t lj = __float_as_uint(q.y);
-  if (track && lj < li && d2 < best_in) {
-    const float ur = eth * 2.5f + llj * 1.3f;
-    if (d2 <= ur * ur && !within2_t(th, index, j)) { best_in = d2; best_j = j; best_t = t; }
+constexpr int kScWarps = 4;            // warps per block
+constexpr uint32_t kScV = 8;           // vertices per warp
+constexpr uint32_t kScCells = 96;      // cells of a union
+constexpr uint32_t kScSlotBits = 27;   // queue entries: vertex << 27 | slot
+constexpr uint32_t kScSlotMask = (1u << kScSlotBits) - 1u;
+struct ScWarp {
+  // the cluster's vertices
+  uint32_t index[kScV], pin[kScV], th_b[kScV], th_n[kScV], th_first[kScV], th_last[kScV];
+  float px[kScV], py[kScV], pz[kScV], xx[kScV], xy[kScV], xz[kScV], ml[kScV], th[kScV], ll[kScV];
+  int32_t cx[kScV], cy[kScV], cz[kScV];
+  unsigned long long best[kScV];         // untangle candidate: distance^2 bits, order
+  // the union's candidates (union_ranges)
+  uint32_t end[kScCells], beg[kScCells];
+  uint8_t box[kScCells];
+  // staged candidates: p and reach, layer, slot
+  float4 cp[36];
+  uint32_t clayer[36], cslot[36];
+  uint32_t q[64];                       // past the scan
+  uint32_t uq[64];                      // untangle candidates past the scan
+  uint4 vq[36];                         // past the gate: pair, star range, contact thickness
+  uint2 bq[64];                         // past the box test: pair, star entry
+  uint2 tq[64];                         // past the owner test
+  uint32_t vv[64];                      // vertex-vertex contacts
+  __device__ __forceinline__ VertCtx ctx(uint32_t i) const {
+    return VertCtx{index[i], pin[i] != 0u, mk(xx[i], xy[i], xz[i]), mk(px[i], py[i], pz[i]), ml[i], th[i], ll[i],
+                   I3{cx[i], cy[i], cz[i]}};
   }
-  return d2 <= mgd * mgd;
+};
+// two-hop list of the cluster's vertex i (see th_find)
+__device__ __forceinline__ bool sc_th_find(const SCArgs& s, const ScWarp& m, uint32_t i, uint32_t b, uint32_t& pos) {
+  // most vertices met in contact belong to another part of the mesh
+  if (b < m.th_first[i] || b > m.th_last[i]) return false;
+  uint32_t at = m.th_b[i];
+  for (uint32_t len = m.th_n[i]; len > 1u;) {
+    const uint32_t half = len >> 1;
+    at += s.th_idx[at + half - 1u] < b ? half : 0u;
+    len -= half;
+  }
+  pos = at;
+  return s.th_idx[at] == b;
+}
+__device__ __forceinline__ bool sc_within2(const SCArgs& s, const ScWarp& m, uint32_t i, uint32_t b) {
+  uint32_t q;
+  return m.index[i] == b || sc_th_find(s, m, i, b, q);
+}
+__device__ __forceinline__ bool near_cell(const I3& a, const int4& b) {
+  return abs(b.x - a.x) <= 1 && abs(b.y - a.y) <= 1 && abs(b.z - a.z) <= 1;
+}
+// The box of cells around the 27-cell neighbourhoods of a cluster, at most
+// kScCells of them: cells [o, o + e).
+struct UnionBox {
+  int32_t ox, oy, oz;
+  uint32_t ex, ey, ez;
+  // place of a cell in the box, ~0 outside
+  __device__ __forceinline__ uint32_t at(const int4& c) const {
+    const uint32_t bx = uint32_t(c.x) - uint32_t(ox), by = uint32_t(c.y) - uint32_t(oy), bz = uint32_t(c.z) - uint32_t(oz);
+    return bx < ex && by < ey && bz < ez ? (bx * ey + by) * ez + bz : ~0u;
+  }
+};
+// The box for all elements of the cluster in `todo` (lanes; element v of lane),
+// or, where that is more than kScCells, for as many as fit; mine: this lane's
+// element is in it.
+template <uint32_t kV>
+__device__ __forceinline__ UnionBox union_box(const I3& cell, uint32_t todo, uint32_t v, uint32_t lane, bool& mine) {
+  const bool in = (todo >> lane) & 1u;
+  int32_t ox = __reduce_min_sync(0xffffffffu, in ? cell.x : INT32_MAX);
+  int32_t oy = __reduce_min_sync(0xffffffffu, in ? cell.y : INT32_MAX);
+  int32_t oz = __reduce_min_sync(0xffffffffu, in ? cell.z : INT32_MAX);
+  int32_t hx = __reduce_max_sync(0xffffffffu, in ? cell.x : INT32_MIN);
+  int32_t hy = __reduce_max_sync(0xffffffffu, in ? cell.y : INT32_MIN);
+  int32_t hz = __reduce_max_sync(0xffffffffu, in ? cell.z : INT32_MIN);
+  mine = in;
+  uint32_t ex = uint32_t(hx) - uint32_t(ox) + 3u, ey = uint32_t(hy) - uint32_t(oy) + 3u,
+           ez = uint32_t(hz) - uint32_t(oz) + 3u;
+  if (ex > kScCells || ey > kScCells || ez > kScCells || ex * ey * ez > kScCells) {
+    const int lead = __ffs(todo) - 1;
+    ox = hx = __shfl_sync(0xffffffffu, cell.x, lead);
+    oy = hy = __shfl_sync(0xffffffffu, cell.y, lead);
+    oz = hz = __shfl_sync(0xffffffffu, cell.z, lead);
+    ex = ey = ez = 3u;
+    mine = false;
+    for (uint32_t w = 0; w < kV; ++w) {
+      const int32_t wx = __shfl_sync(0xffffffffu, cell.x, w), wy = __shfl_sync(0xffffffffu, cell.y, w),
+                    wz = __shfl_sync(0xffffffffu, cell.z, w);
+      if (!((todo >> w) & 1u)) continue;
+      const int32_t nx = min(ox, wx), ny = min(oy, wy), nz = min(oz, wz);
+      const int32_t mx = max(hx, wx), my = max(hy, wy), mz = max(hz, wz);
+      const uint32_t fx = uint32_t(mx) - uint32_t(nx) + 3u, fy = uint32_t(my) - uint32_t(ny) + 3u,
+                     fz = uint32_t(mz) - uint32_t(nz) + 3u;
+      if (fx > kScCells || fy > kScCells || fz > kScCells || fx * fy * fz > kScCells) continue;
+      ox = nx; oy = ny; oz = nz;
+      hx = mx; hy = my; hz = mz;
+      ex = fx; ey = fy; ez = fz;
+      mine = mine || v == w;
+    }
+  }
+  return UnionBox{int32_t(uint32_t(ox) - 1u), int32_t(uint32_t(oy) - 1u), int32_t(uint32_t(oz) - 1u), ex, ey, ez};
+}
+// The candidates of a box's cells, flattened over its non-empty buckets: for
+// the r-th, end[r] = candidates up to and including it, beg[r] = slot of its
+// first minus the candidates before it, box[r] = the cell's place in the box
+// (a bucket may hold other cells' elements too, and may come up for several
+// cells; an element counts where its own cell is the bucket's).  skip(begin,
+// end) returns where a bucket's candidates start.  Returns their number.
+template <class F>
+__device__ __forceinline__ uint32_t union_ranges(const UnionBox& ub, uint32_t table, const uint32_t* starts,
+                                                 uint32_t* end, uint32_t* beg_out, uint8_t* box, uint32_t lane,
+                                                 F&& skip) {
+  const uint32_t lt_mask = (1u << lane) - 1u;
+  uint32_t total = 0, kept = 0;
+  const uint32_t eyz = ub.ey * ub.ez, vol = ub.ex * eyz;
+  __syncwarp();
+  for (uint32_t q0 = 0; q0 < vol; q0 += 32u) {
+    const uint32_t q = q0 + lane;
+    uint32_t beg = 0, cnt = 0;
+    if (q < vol) {
+      const uint32_t qx = q / eyz, r = q - qx * eyz, qy = r / ub.ez;
+      const uint32_t h = hash3(int32_t(uint32_t(ub.ox) + qx), int32_t(uint32_t(ub.oy) + qy),
+                               int32_t(uint32_t(ub.oz) + r - qy * ub.ez), table);
+      const uint32_t en = starts[h + 1];
+      beg = skip(starts[h], en);
+      cnt = en - beg;
+    }
+    uint32_t incl = cnt;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+      if (int(lane) >= o) incl += u;
+    }
+    const uint32_t some = __ballot_sync(0xffffffffu, cnt != 0u);
+    if (cnt) {
+      const uint32_t r = kept + __popc(some & lt_mask);
+      end[r] = total + incl;
+      beg_out[r] = beg - (total + incl - cnt);
+      box[r] = uint8_t(q);
+    }
+    kept += __popc(some);
+    total += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  __syncwarp();
+  return total;
 }
 
-// Contact work for one candidate that passed sc_filter
-// (shaders/self_collision.wgsl:392-670), part 1: the vertex-vertex contact
-// and the vertex-triangle gate.  Returns true with the star range of j when
-// j's incident triangles must be tested (part 2, vt_entry).
-__device__ __forceinline__ bool sc_work_vv(const SCArgs& s, const VertCtx& c, const TwoHop& th, uint32_t slot,
-                                           uint32_t& st_b, uint32_t& st_e, float4& rec0, float4& rec1) {
-  const uint32_t index = c.index;
+// Reach of a vertex in the scan.  A pair matters only within
+// max(eth, vtb) <= vtb = eth + 1.3 llj + mli + mlj (the tests of sc_gate) with
+// eth <= thi + thj + 0.06 lli, so within reach_i + reach_j; a slack of 1e-5
+// covers the rounding on both sides.  Not finite: within reach of everything.
+__device__ __forceinline__ float sc_reach(float th, float ll_part, float ml) {
+  const float r = (fmaxf(th, 0.f) + ll_part + ml) * 1.00001f + 1e-9f;
+  return r < 1e18f ? r : 1e18f;
+}
+
+// Exact tests of one pair (shaders/self_collision.wgsl:356-470): the cluster's
+// vertex i, candidate slot.  vv: the vertex-vertex contact math must run
+// (vv_contact); true with the star range of the candidate and the contact
+// thickness when its incident triangles must be tested.
+__device__ __forceinline__ bool sc_gate(const SCArgs& s, const ScWarp& m, uint32_t i, uint32_t slot, bool& vv,
+                                        uint32_t& st_b, uint32_t& st_n, float& out_eth) {
+  vv = false;
+  const VertCtx c = m.ctx(i);
   const int4 jc = s.vs_c[slot];
   const uint32_t j = (uint32_t)jc.w;
-  const float wi = c.wi;
-  const bool pin_i = c.pin_i;
-  const V3 pi = c.pi;
-  const float mli = c.mli, thi = c.thi, lli = c.lli;
-  const uint32_t li = c.li;
-  const bool untangle = c.untangle;
-  int32_t* acc = s.acc;
   const float4 pj4 = s.vs_p[slot];
   const float4 q = s.vs_q[slot];
-  const V3 pj = mk(pj4);
-  const V3 dvv = pi - pj;
+  if (j == c.index || !near_cell(c.cell, jc)) return false;
+  const V3 dvv = c.pi - mk(pj4);
   const float d2 = dot(dvv, dvv);
-  const float thj = pj4.w, llj = q.x;
-  const float eth = fmaxf(thi + thj, fminf(lli, llj) * 0.06f);
-  const uint32_t lj = __float_as_uint(q.y);
-  const float dvl = sqrtf(fmaxf(d2, 0.0f));
+  const float llj = q.x;
+  const float eth = fmaxf(c.thi + pj4.w, fminf(c.lli, llj) * 0.06f);
+  const float mgd = eth + (c.lli + llj) * 1.3f;
+  const float vtb = eth + llj * 1.3f + c.mli + q.w;
+  const bool near_v = d2 < eth * eth, near_t = d2 <= vtb * vtb;
+  if (!(d2 <= mgd * mgd && (near_v || near_t))) return false;
   // one search of i's two-hop list serves both tests on j: near_folded
   // (:268-293) and, below, within_two_hops (:243-264); j != index here
   uint32_t thq = 0;
-  const bool j_in2 = th_find(th, j, thq);
-  if (j_in2 && !(dvl < th.rest[thq] * 0.5f)) return false;
-  const V3 pjo = mk(s.x4[j]);
-  const float wj = q.z;
-  const bool both = wj > 0.0f;
-  const float eth2 = eth * eth;
-  // 1. vertex-vertex
-  if (!pin_i && (!both || index < j)) {
-    if (d2 < eth2 && d2 > kEps * kEps) {
-      bool utv = false;
-      if (untangle && li != lj) {
-        const V3 ni = mk(s.nrm[index]), nj = mk(s.nrm[j]);
-        const float nil = length(ni), njl = length(nj);
-        if (li > lj) {
-          if (njl > 0.5f) {
-            const V3 nju = nj / njl;
-            const bool allow = (wj <= 0.0f) || (nil <= 0.5f) || (dot(ni / fmaxf(nil, kEps), nju) > 0.0f);
-            utv = allow && (dot(dvv, nju) < 0.0f);
-          }
-        } else if (both && nil > 0.5f) {
-          const V3 niu = ni / nil;
-          const bool allow = (njl <= 0.5f) || (dot(nj / fmaxf(njl, kEps), niu) > 0.0f);
-          utv = allow && (dot(-dvv, niu) < 0.0f);
-        }
-      }
-      if (!utv) {
-        const V3 nn = dvv / dvl;
-        const float pen = eth - dvl;
-        const float ws = wi + wj;
-        if (ws > kEps) {
-          if (wj <= 0.0f) {
-            add_pin(acc, index, nn * pen + (pj - pjo) * 0.5f);
-          } else {
-            const V3 disp = nn * (pen * 0.5f);
-            add_disp(acc, index, disp * (wi / ws));
-            add_disp(acc, j, (-disp) * (wj / ws));
-          }
-        }
-      }
-    }
-  }
-  // 2. vertex-triangle
-  const float mlj = q.w;
-  const float vtb = eth + llj * 1.3f + mli + mlj;
-  if (!(d2 <= vtb * vtb) || j_in2) return false;
-  {
-    // Every triangle of j's star is skipped by its own swept-box test
-    // (smin > tmax or smax < tmin on an axis) when the widest possible swept
-    // box of i, over the star's motion range plus a 10 um rounding margin,
-    // misses the star's box: skipping the whole star is then exact.
-    const float4 b0 = s.sbox[3 * size_t(j)], b1 = s.sbox[3 * size_t(j) + 1], b2 = s.sbox[3 * size_t(j) + 2];
-    const V3 xi = c.xi;
-    const float sl = 1e-5f;
-    const float rl[3] = {xi.x + b0.w - sl, xi.y + b1.w - sl, xi.z + b2.w - sl};
-    const float rh[3] = {xi.x + b2.x + sl, xi.y + b2.y + sl, xi.z + b2.z + sl};
-    const float pa[3] = {pi.x, pi.y, pi.z};
-    const float lo[3] = {b0.x, b0.y, b0.z}, hi[3] = {b1.x, b1.y, b1.z};
+  const bool j_in2 = sc_th_find(s, m, i, j, thq);
+  if (j_in2 && !(sqrtf(fmaxf(d2, 0.0f)) < s.th_rest[thq] * 0.5f)) return false;
+  vv = !c.pin_i && (!(q.z > 0.0f) || c.index < j) && near_v && d2 > kEps * kEps;
+  if (!near_t || j_in2) return false;
+  // Every triangle of j's star is skipped by its own swept-box test
+  // (smin > tmax or smax < tmin on an axis) when the widest possible swept
+  // box of i, over the star's motion range plus a 10 um rounding margin,
+  // misses the star's box: skipping the whole star is then exact.
+  const float4 b0 = s.sbox[3 * size_t(j)], b1 = s.sbox[3 * size_t(j) + 1], b2 = s.sbox[3 * size_t(j) + 2];
+  const V3 xi = c.xi, pi = c.pi;
+  const float sl = 1e-5f;
+  const float rl[3] = {xi.x + b0.w - sl, xi.y + b1.w - sl, xi.z + b2.w - sl};
+  const float rh[3] = {xi.x + b2.x + sl, xi.y + b2.y + sl, xi.z + b2.z + sl};
+  const float pa[3] = {pi.x, pi.y, pi.z};
+  const float lo[3] = {b0.x, b0.y, b0.z}, hi[3] = {b1.x, b1.y, b1.z};
 #pragma unroll
-    for (int ax = 0; ax < 3; ++ax) {
-      const float smin_lb = fminf(rl[ax], pa[ax]) - eth - sl;
-      const float smax_ub = fmaxf(rh[ax], pa[ax]) + eth + sl;
-      if (smin_lb > hi[ax] || smax_ub < lo[ax]) return false;
-    }
+  for (int ax = 0; ax < 3; ++ax) {
+    const float smin_lb = fminf(rl[ax], pa[ax]) - eth - sl;
+    const float smax_ub = fmaxf(rh[ax], pa[ax]) + eth + sl;
+    if (smin_lb > hi[ax] || smax_ub < lo[ax]) return false;
   }
   st_b = s.star_off[j];
-  st_e = s.star_off[j + 1];
-  // what the triangle filter needs of j: p, contact thickness, x, index
-  rec0 = make_float4(pj.x, pj.y, pj.z, eth);
-  rec1 = make_float4(pjo.x, pjo.y, pjo.z, __uint_as_float(j));
-  return st_e > st_b;
+  st_n = s.star_off[j + 1] - st_b;
+  out_eth = eth;
+  return st_n > 0u;
+}
+// One untangle candidate of the cluster's vertex i (:377-383): its key
+// (distance^2 bits, visiting order), or all ones.
+__device__ __forceinline__ unsigned long long sc_untangle_key(const SCArgs& s, const ScWarp& m, uint32_t i,
+                                                              uint32_t slot) {
+  const int4 jc = s.vs_c[slot];
+  const float4 pj4 = s.vs_p[slot];
+  const float llj = s.vs_q[slot].x;
+  const I3 cell{m.cx[i], m.cy[i], m.cz[i]};
+  const V3 dvv = mk(m.px[i], m.py[i], m.pz[i]) - mk(pj4);
+  const float d2 = dot(dvv, dvv);
+  const float eth = fmaxf(m.th[i] + pj4.w, fminf(m.ll[i], llj) * 0.06f);
+  const float ur = eth * 2.5f + llj * 1.3f;
+  if (!near_cell(cell, jc) || !(d2 < 1e20f) || !(d2 <= ur * ur) || sc_within2(s, m, i, (uint32_t)jc.w)) return ~0ull;
+  const uint32_t k = uint32_t((jc.x - cell.x + 1) * 9 + (jc.y - cell.y + 1) * 3 + (jc.z - cell.z + 1));
+  return (unsigned long long)__float_as_uint(d2) << 32 | (k << kScSlotBits | slot);
 }
 
-// Part 2: one (candidate j, incident triangle) pair, star entry `st` of j
-// (shaders/self_collision.wgsl:477-667).  kHeavy = false runs the cheap tests
-// (ownership, swept bounds, two-hop exclusion) on j's values cached by
-// sc_work_vv (rec0 = p_j, contact thickness; rec1 = x_j, j) and returns
-// whether the pair needs the contact math; kHeavy = true reloads j and runs
-// the whole pair.  Each pair is independent (its output goes through the
-// order-free integer accumulators).
-template <bool kHeavy>
-__device__ __forceinline__ bool vt_entry(const SCArgs& s, const VertCtx& c, const TwoHop& th, uint32_t slot,
-                                         uint32_t st, float4 rec0 = float4(), float4 rec1 = float4()) {
-  const uint32_t index = c.index;
-  const float wi = c.wi;
-  const bool pin_i = c.pin_i;
-  const V3 xi = c.xi, pi = c.pi;
-  const float mli = c.mli, thi = c.thi, lli = c.lli;
-  const I3 cell = c.cell;
-  const uint32_t li = c.li;
-  const bool untangle = c.untangle;
-  int32_t* acc = s.acc;
-  V3 pj, pjo;
-  uint32_t j, lj = 0u;
-  float eth, wj = 0.f;
-  if (kHeavy) {
-    j = (uint32_t)s.vs_c[slot].w;
-    const float4 pj4 = s.vs_p[slot];
-    const float4 q = s.vs_q[slot];
-    pj = mk(pj4);
-    eth = fmaxf(thi + pj4.w, fminf(lli, q.x) * 0.06f);
-    lj = __float_as_uint(q.y);
-    pjo = mk(s.x4[j]);
-    wj = q.z;
-  } else {
-    pj = mk(rec0);
-    eth = rec0.w;
-    pjo = mk(rec1);
-    j = __float_as_uint(rec1.w);
+// Sum of d into vertex v's displacement (add_disp) for the lanes with `on`,
+// called by the whole warp.  The lanes of a batch mostly share a few v, whose
+// contributions are summed in the warp first: integer sums, so the order is
+// free.
+__device__ __forceinline__ void add_disp_shared(int32_t* acc, uint32_t v, V3 d, bool on) {
+  const uint32_t peers = __match_any_sync(0xffffffffu, on ? v : 0xFFFFFFFFu);
+  if (!on) return;
+  const int32_t x = __reduce_add_sync(peers, to_fixed(d.x));
+  const int32_t y = __reduce_add_sync(peers, to_fixed(d.y));
+  const int32_t z = __reduce_add_sync(peers, to_fixed(d.z));
+  if (int(threadIdx.x & 31u) == __ffs(peers) - 1) {
+    int32_t* a = acc + (size_t)v * A_N;
+    atomicAdd(&a[A_DX], x);
+    atomicAdd(&a[A_DY], y);
+    atomicAdd(&a[A_DZ], z);
+    atomicAdd((uint32_t*)&a[A_CNT], uint32_t(__popc(peers)));
   }
-  const float eth2 = eth * eth;
+}
 
-  const uint2 pr = s.star_idx[st];
-  const uint32_t v0 = pr.x, v1 = pr.y;
-  if (v0 == index || v1 == index) return false;
-  const float4 q0 = s.p4[v0], q1 = s.p4[v1];
-  const V3 pv0 = mk(q0), pv1 = mk(q1);
-  // ownership (:486-500): the triangle is tested from its in-range vertex of
-  // smallest index, so only a vertex below j can take it away; the in-range
-  // test of v0 (v1) runs, and loads its data, only when v0 < j (v1 < j)
-  if (j > v0) {
-    const V3 d0 = pi - pv0;
-    const float ll0 = s.local_len[v0];
-    const float et0 = fmaxf(thi + q0.w, fminf(lli, ll0) * 0.06f);
-    const float b0 = et0 + ll0 * 1.3f + mli + s.mlen[v0];
-    const int4 c0 = s.vcell[v0];
-    if (abs(c0.x - cell.x) <= 1 && abs(c0.y - cell.y) <= 1 && abs(c0.z - cell.z) <= 1 && (dot(d0, d0) <= b0 * b0))
-      return false;
+// The vertex-vertex contact (shaders/self_collision.wgsl:405-460) of vertex
+// `index` (not pinned) and candidate slot `slot`, which are closer than their
+// contact thickness.
+__device__ __forceinline__ void vv_contact(const SCArgs& s, uint32_t index, uint32_t slot) {
+  const float4 pi4 = s.p4[index];
+  const float wi = s.x4[index].w;
+  const uint32_t j = (uint32_t)s.vs_c[slot].w;
+  const float4 pj4 = s.vs_p[slot];
+  const float4 q = s.vs_q[slot];
+  const V3 pj = mk(pj4), dvv = mk(pi4) - pj;
+  const float eth = fmaxf(pi4.w + pj4.w, fminf(s.local_len[index], q.x) * 0.06f);
+  const float dvl = sqrtf(fmaxf(dot(dvv, dvv), 0.0f));
+  const float wj = q.z;
+  const bool both = wj > 0.0f;
+  int32_t* acc = s.acc;
+  bool utv = false;
+  if (s.untangle != 0) {
+    const uint32_t li = layer_of(s.v4, index), lj = __float_as_uint(q.y);
+    if (li != lj) {
+      const V3 ni = mk(s.nrm[index]), nj = mk(s.nrm[j]);
+      const float nil = length(ni), njl = length(nj);
+      if (li > lj) {
+        if (njl > 0.5f) {
+          const V3 nju = nj / njl;
+          const bool allow = (wj <= 0.0f) || (nil <= 0.5f) || (dot(ni / fmaxf(nil, kEps), nju) > 0.0f);
+          utv = allow && (dot(dvv, nju) < 0.0f);
+        }
+      } else if (both && nil > 0.5f) {
+        const V3 niu = ni / nil;
+        const bool allow = (njl <= 0.5f) || (dot(nj / fmaxf(njl, kEps), niu) > 0.0f);
+        utv = allow && (dot(-dvv, niu) < 0.0f);
+      }
+    }
   }
-  if (j > v1) {
-    const V3 d1 = pi - pv1;
-    const float ll1 = s.local_len[v1];
-    const float et1 = fmaxf(thi + q1.w, fminf(lli, ll1) * 0.06f);
-    const float b1 = et1 + ll1 * 1.3f + mli + s.mlen[v1];
-    const int4 c1 = s.vcell[v1];
-    if (abs(c1.x - cell.x) <= 1 && abs(c1.y - cell.y) <= 1 && abs(c1.z - cell.z) <= 1 && (dot(d1, d1) <= b1 * b1))
-      return false;
+  if (utv) return;
+  const V3 nn = dvv / dvl;
+  const float pen = eth - dvl;
+  const float ws = wi + wj;
+  if (ws > kEps) {
+    if (wj <= 0.0f) {
+      add_pin(acc, index, nn * pen + (pj - mk(s.x4[j])) * 0.5f);
+    } else {
+      const V3 disp = nn * (pen * 0.5f);
+      add_disp(acc, index, disp * (wi / ws));
+      add_disp(acc, j, (-disp) * (wj / ws));
+    }
   }
-  const float4 o0 = s.x4[v0], o1 = s.x4[v1];
-  const V3 pv0o = mk(o0), pv1o = mk(o1);
-  const float wv0 = o0.w, wv1 = o1.w;
-  const V3 tmove = (((pj - pjo) + (pv0 - pv0o)) + (pv1 - pv1o)) / 3.0f;
-  const bool tpin = (wj <= 0.0f) || (wv0 <= 0.0f) || (wv1 <= 0.0f);
-  const V3 rel = xi + tmove;
+}
+
+// One (candidate j, incident triangle) pair, star entry `st` of j
+// (shaders/self_collision.wgsl:477-667).  The cheap tests (swept bounds,
+// ownership, two-hop exclusion; any order gives the same outcome) come first,
+// in vt_box and vt_owner; a pair that passes both needs the contact math,
+// vt_contact.  Each pair is independent (its output goes through the
+// order-free integer accumulators).
+//
+// vt_box: the swept box of the vertex against the triangle's, on the star
+// entry's record and the contact thickness eth of (i, j)
+__device__ __forceinline__ bool vt_box(const SCArgs& s, const ScWarp& m, uint32_t i, float eth, uint32_t st) {
+  const float4 tlo = s.st_lo[st], thi = s.st_hi[st];
+  const float mz = s.st_mz[st];
+  const V3 pi = mk(m.px[i], m.py[i], m.pz[i]);
+  const V3 rel = mk(m.xx[i], m.xy[i], m.xz[i]) + mk(tlo.w, thi.w, mz);
   const V3 E = mk(eth, eth, eth);
   const V3 smin = vmin(rel, pi) - E, smax = vmax(rel, pi) + E;
-  const V3 tmin = vmin(vmin(pj, pv0), pv1), tmax = vmax(vmax(pj, pv0), pv1);
-  if (smin.x > tmax.x || smin.y > tmax.y || smin.z > tmax.z || smax.x < tmin.x || smax.y < tmin.y ||
-      smax.z < tmin.z)
-    return false;
-  if (within2_t(th, index, v0) || within2_t(th, index, v1)) return false;
-  if (!kHeavy) return true;
+  return !(smin.x > thi.x || smin.y > thi.y || smin.z > thi.z || smax.x < tlo.x || smax.y < tlo.y || smax.z < tlo.z);
+}
+// ownership (:486-500): the triangle is tested from its in-range vertex of
+// smallest index, so only a vertex below j can take it away; then the two-hop
+// exclusion
+__device__ __forceinline__ bool vt_owner(const SCArgs& s, const ScWarp& m, uint32_t i, uint32_t j, uint32_t st) {
+  const uint2 pr = s.star_idx[st];
+  const uint32_t index = m.index[i];
+  if (pr.x == index || pr.y == index) return false;
+  const V3 pi = mk(m.px[i], m.py[i], m.pz[i]);
+  const float thi = m.th[i], lli = m.ll[i], mli = m.ml[i];
+  const I3 cell{m.cx[i], m.cy[i], m.cz[i]};
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const uint32_t v = e ? pr.y : pr.x;
+    if (j > v) {
+      const float4 q = s.p4[v];
+      const V3 d = pi - mk(q);
+      const float ll = s.local_len[v];
+      const float et = fmaxf(thi + q.w, fminf(lli, ll) * 0.06f);
+      const float b = et + ll * 1.3f + mli + s.mlen[v];
+      if (dot(d, d) <= b * b && near_cell(cell, s.vcell[v])) return false;
+    }
+  }
+  return !sc_within2(s, m, i, pr.x) && !sc_within2(s, m, i, pr.y);
+}
+
+// The contact math of a pair that passed the cheap tests: vertex `index`,
+// candidate slot `slot`, star entry `st`; called by the whole warp, `on` lanes
+// work.  What both contact forms end in, a displacement tp shared by the four
+// vertices, is added after the branches.
+__device__ __forceinline__ void vt_contact(const SCArgs& s, bool on, uint32_t index, uint32_t slot, uint32_t st) {
+  int32_t* acc = s.acc;
+  bool push = false;
+  V3 tp = mk(0.f, 0.f, 0.f), bw = mk(0.f, 0.f, 0.f);
+  float wi = 0.f, wj = 0.f, wv0 = 0.f, wv1 = 0.f, wtot = 1.f;
+  uint32_t j = 0, v0 = 0, v1 = 0;
+  if (on) {
+  const float4 xi4 = s.x4[index], pi4 = s.p4[index];
+  wi = xi4.w;
+  const bool pin_i = wi <= 0.0f;
+  const V3 xi = mk(xi4), pi = mk(pi4);
+  const uint32_t li = layer_of(s.v4, index);
+  const bool untangle = s.untangle != 0;
+  j = (uint32_t)s.vs_c[slot].w;
+  const float4 pj4 = s.vs_p[slot];
+  const float4 q = s.vs_q[slot];
+  const uint2 pr = s.star_idx[st];
+  v0 = pr.x;
+  v1 = pr.y;
+  const V3 tmove = mk(s.st_lo[st].w, s.st_hi[st].w, s.st_mz[st]);
+  const V3 pj = mk(pj4);
+  const float eth = fmaxf(pi4.w + pj4.w, fminf(s.local_len[index], q.x) * 0.06f);
+  const uint32_t lj = __float_as_uint(q.y);
+  wj = q.z;
+  const float eth2 = eth * eth;
+  const V3 pv0 = mk(s.p4[v0]), pv1 = mk(s.p4[v1]);
+  wv0 = s.x4[v0].w;
+  wv1 = s.x4[v1].w;
+  const bool tpin = (wj <= 0.0f) || (wv0 <= 0.0f) || (wv1 <= 0.0f);
+  const V3 rel = xi + tmove;
   const V3 mv = pi - rel;
   const float msq = dot(mv, mv);
   float ht = 1.0f, hu = 0.0f, hv = 0.0f;
@@ -750,18 +922,16 @@ __device__ __forceinline__ bool vt_entry(const SCArgs& s, const VertCtx& c, cons
       } else {
         const V3 bc = mk(clampf(1.0f - hu - hv, 0.0f, 1.0f), clampf(hu, 0.0f, 1.0f), clampf(hv, 0.0f, 1.0f));
         const float wt = bc.x * bc.x * wj + bc.y * bc.y * wv0 + bc.z * bc.z * wv1;
-        const float wtot = wi + wt;
+        wtot = wi + wt;
         if (wtot > kEps) {
           add_ccd(acc, index, tccd * (wi / wtot), false);
           if (wj > 0.0f) add_ccd(acc, j, (-tccd) * (bc.x * wj / wtot), false);
           if (wv0 > 0.0f) add_ccd(acc, v0, (-tccd) * (bc.y * wv0 / wtot), false);
           if (wv1 > 0.0f) add_ccd(acc, v1, (-tccd) * (bc.z * wv1 / wtot), false);
           if (pcs > kEps) {
-            const V3 tp = ns * (pcs * 0.6f);
-            add_disp(acc, index, tp * (wi / wtot));
-            if (wj > 0.0f) add_disp(acc, j, (-tp) * (bc.x * wj / wtot));
-            if (wv0 > 0.0f) add_disp(acc, v0, (-tp) * (bc.y * wv0 / wtot));
-            if (wv1 > 0.0f) add_disp(acc, v1, (-tp) * (bc.z * wv1 / wtot));
+            tp = ns * (pcs * 0.6f);
+            bw = bc;
+            push = true;
           }
         }
       }
@@ -794,166 +964,251 @@ __device__ __forceinline__ bool vt_entry(const SCArgs& s, const VertCtx& c, cons
           add_pin(acc, index, nvt * pvt + tmove * 0.5f);
         } else {
           const float wt = bary.x * bary.x * wj + bary.y * bary.y * wv0 + bary.z * bary.z * wv1;
-          const float wtot = wi + wt;
+          wtot = wi + wt;
           if (wtot > kEps) {
-            const V3 tp = nvt * (pvt * 0.6f);
-            add_disp(acc, index, tp * (wi / wtot));
-            if (wj > 0.0f) add_disp(acc, j, (-tp) * (bary.x * wj / wtot));
-            if (wv0 > 0.0f) add_disp(acc, v0, (-tp) * (bary.y * wv0 / wtot));
-            if (wv1 > 0.0f) add_disp(acc, v1, (-tp) * (bary.z * wv1 / wtot));
+            tp = nvt * (pvt * 0.6f);
+            bw = bary;
+            push = true;
           }
         }
       }
     }
   }
-  return true;
+  }
+  add_disp_shared(acc, index, tp * (wi / wtot), push);
+  if (push) {
+    if (wj > 0.0f) add_disp(acc, j, (-tp) * (bw.x * wj / wtot));
+    if (wv0 > 0.0f) add_disp(acc, v0, (-tp) * (bw.y * wv0 / wtot));
+    if (wv1 > 0.0f) add_disp(acc, v1, (-tp) * (bw.z * wv1 / wtot));
+  }
 }
 
-__global__ void __launch_bounds__(256, 4) k_sc_solve(SCArgs s) {
-  __shared__ uint32_t sh_start[8][28], sh_end[8][28], sh_beg[8][28];
-  __shared__ uint32_t sh_th[8][kTwoHopCache];
-  __shared__ float sh_thr[8][kTwoHopCache];
-  __shared__ uint32_t sh_q[8][32 * kRounds];
-  __shared__ uint32_t pr_slot[8][32], pr_sb[8][32], pr_ex[8][32];  // survivors' star ranges
-  __shared__ uint32_t tq_slot[8][64], tq_st[8][64];                 // (candidate, triangle) pairs
-  __shared__ float4 pr_rec0[8][32], pr_rec1[8][32];                 // survivors' cached values
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t index = blockIdx.x * 8u + warp;
-  if (index >= s.n) return;  // whole warp
-  VertCtx c;
-  c.index = index;
-  const float4 xi4 = s.x4[index], pi4 = s.p4[index];
-  c.wi = xi4.w;
-  c.pin_i = c.wi <= 0.0f;
-  c.xi = mk(xi4);
-  c.pi = mk(pi4);
-  c.mli = s.mlen[index];
-  if (c.pin_i && c.mli < kEps) return;  // whole warp
-  const TwoHop th = stage_two_hop(s.th_off, s.th_idx, s.th_rest, index, sh_th[warp], sh_thr[warp], lane);
-  c.thi = pi4.w;
-  c.lli = s.local_len[index];
-  {
-    const int4 vc = s.vcell[index];
-    c.cell = I3{vc.x, vc.y, vc.z};
-  }
-  c.li = layer_of(s.v4, index);
-  c.untangle = s.untangle != 0;
-  c.track = c.untangle && !c.pin_i && c.li > 0u;
-  // bucket ranges of the 27 neighbour cells, lane k = (dx+1)*9 + (dy+1)*3 + (dz+1)
-  uint32_t cnt = 0, beg = 0;
-  if (lane < 27) {
-    const uint32_t h = hash3(c.cell.x - 1 + lane / 9, c.cell.y - 1 + (lane / 3) % 3, c.cell.z - 1 + lane % 3, s.table);
-    beg = s.cs[h];
-    cnt = s.cs[h + 1] - beg;
-  }
-  uint32_t incl = cnt;
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  if (lane < 27) {
-    sh_start[warp][lane] = incl - cnt;
-    sh_end[warp][lane] = incl;
-    sh_beg[warp][lane] = beg;
-  }
-  __syncwarp();
-  const uint32_t total = __shfl_sync(0xffffffffu, incl, 26);
-  float best_in = 1e20f;
-  uint32_t best_j = 0xFFFFFFFFu, best_t = 0xFFFFFFFFu;
-  int k = 0;
-  uint32_t* queue = sh_q[warp];
+__global__ void __launch_bounds__(32 * kScWarps, 7) k_sc_solve(const __grid_constant__ SCArgs s) {
+  __shared__ ScWarp sh[kScWarps];
+  const uint32_t lane = threadIdx.x & 31u;
+  ScWarp& m = sh[threadIdx.x >> 5];
   const uint32_t lt_mask = (1u << lane) - 1u;
-  uint32_t tqn = 0;
-  for (uint32_t chunk = 0; chunk < total; chunk += 32u * kRounds) {
-    // phase 1: cheap filters on 32 x kRounds candidates, survivors compacted
-    uint32_t qn = 0;
-    for (uint32_t r = 0; r < kRounds; ++r) {
-      const uint32_t t = chunk + r * 32u + lane;
+  const uint32_t at = (blockIdx.x * kScWarps + (threadIdx.x >> 5)) * kScV;
+  if (at >= s.n) return;  // whole warp
+  // a lane's vertex, and which of the 32 / kScV candidates at a time it tests
+  const uint32_t v = lane % kScV, sub = lane / kScV;
+  constexpr uint32_t kSub = 32u / kScV;
+  // ---- the cluster
+  const uint32_t index = at + v < s.n ? s.order[at + v] : 0xFFFFFFFFu;
+  bool live = index != 0xFFFFFFFFu;
+  V3 pi = mk(0.f, 0.f, 0.f);
+  float reach = 0.f, treach = 0.f, best_in = -1.f;
+  uint32_t layer = 0;
+  I3 cell{0, 0, 0};
+  if (live) {
+    const float4 xi4 = s.x4[index], pi4 = s.p4[index];
+    const float ml = s.mlen[index], ll = s.local_len[index];
+    const bool pin = xi4.w <= 0.0f;
+    live = !(pin && ml < kEps);
+    const int4 vc = s.vcell[index];
+    cell = I3{vc.x, vc.y, vc.z};
+    pi = mk(pi4);
+    reach = sc_reach(pi4.w, 0.06f * ll, ml);
+    treach = sc_reach(2.5f * pi4.w, 2.5f * 0.06f * ll, 0.f);
+    layer = layer_of(s.v4, index);
+    if (s.untangle && !pin && layer > 0u) best_in = 1e20f;  // tracks an untangle candidate
+    const uint32_t tb = s.th_off[index], tn = s.th_off[index + 1] - tb;
+    m.index[v] = index;
+    m.pin[v] = pin ? 1u : 0u;
+    m.th_b[v] = tb;
+    m.th_n[v] = tn;
+    m.th_first[v] = tn ? s.th_idx[tb] : 1u;
+    m.th_last[v] = tn ? s.th_idx[tb + tn - 1u] : 0u;
+    m.px[v] = pi.x; m.py[v] = pi.y; m.pz[v] = pi.z;
+    m.xx[v] = xi4.x; m.xy[v] = xi4.y; m.xz[v] = xi4.z;
+    m.ml[v] = ml; m.th[v] = pi4.w; m.ll[v] = ll;
+    m.cx[v] = cell.x; m.cy[v] = cell.y; m.cz[v] = cell.z;
+  }
+  m.best[v] = ~0ull;
+  uint32_t todo = __ballot_sync(0xffffffffu, live);
+  uint32_t max_layer = 0;  // of the tracking lanes: candidates of this layer or above interest none of them
+  {
+    const uint32_t l = live && best_in > 0.f ? layer : 0u;
+    max_layer = __reduce_max_sync(0xffffffffu, l);
+  }
+  uint32_t qn = 0, uqn = 0, vqn = 0, bqn = 0, tqn = 0, vvn = 0;  // queue lengths
+  uint32_t pos = 0, total = 0, cn = 0, k = 0;                      // scan position, staged candidates
+  bool mine = false, drain = false;
+  UnionBox ub{0, 0, 0, 0, 0, 0};
+  float4 blo = make_float4(0.f, 0.f, 0.f, 0.f);
+  V3 bhi = pi;
+  for (;;) {
+    __syncwarp();
+    if (tqn >= 32u || (drain && tqn && !bqn && !vqn && !qn)) {  // 5
+      const uint32_t nb = min(tqn, 32u);
+      tqn -= nb;
+      const bool on = lane < nb;
+      const uint2 e = on ? m.tq[tqn + lane] : make_uint2(0u, 0u);
+      vt_contact(s, on, on ? m.index[e.x >> kScSlotBits] : 0u, e.x & kScSlotMask, e.y);
+      continue;
+    }
+    if (vvn >= 32u || (drain && vvn && !qn)) {
+      const uint32_t nb = min(vvn, 32u);
+      vvn -= nb;
+      if (lane < nb) {
+        const uint32_t e = m.vv[vvn + lane];
+        vv_contact(s, m.index[e >> kScSlotBits], e & kScSlotMask);
+      }
+      continue;
+    }
+    if (bqn >= 32u || (drain && bqn && !vqn && !qn)) {  // 4
+      const uint32_t nb = min(bqn, 32u);
+      bqn -= nb;
       bool pass = false;
-      uint32_t slot = 0;
-      if (t < total) {
-        while (t >= sh_end[warp][k]) ++k;
-        slot = sh_beg[warp][k] + (t - sh_start[warp][k]);
-        pass = sc_filter(s, c, th, slot, c.cell.x - 1 + k / 9, c.cell.y - 1 + (k / 3) % 3, c.cell.z - 1 + k % 3, t,
-                         best_in, best_j, best_t);
+      uint2 e = make_uint2(0u, 0u);
+      if (lane < nb) {
+        e = m.bq[bqn + lane];
+        const uint32_t j = (uint32_t)s.vs_c[e.x & kScSlotMask].w;
+        pass = vt_owner(s, m, e.x >> kScSlotBits, j, e.y);
+        if (pass && s.rec_vt) {
+          const uint2 tv = s.star_idx[e.y];
+          record_vt(s, m.index[e.x >> kScSlotBits], j, tv.x, tv.y);
+        }
       }
       const uint32_t b = __ballot_sync(0xffffffffu, pass);
-      if (pass) queue[qn + __popc(b & lt_mask)] = slot;
-      qn += __popc(b);
+      if (pass) m.tq[tqn + __popc(b & lt_mask)] = e;
+      tqn += __popc(b);
+      continue;
     }
-    __syncwarp();
-    // phase 2: vertex-vertex work on the survivors, 32 at a time; each
-    // survivor's incident triangles become (survivor, star entry) pairs
-    for (uint32_t base = 0; base < qn; base += 32u) {
-      const uint32_t q = base + lane;
-      uint32_t sb = 0, se = 0;
-      float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0;
-      const uint32_t slot = q < qn ? queue[q] : 0u;
-      const bool vt = q < qn && sc_work_vv(s, c, th, slot, sb, se, r0, r1);
-      const uint32_t cnt = vt ? se - sb : 0u;
-      uint32_t incl = cnt;
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      const uint32_t npairs = __shfl_sync(0xffffffffu, incl, 31);
-      pr_slot[warp][lane] = slot;
-      pr_sb[warp][lane] = sb;
-      pr_ex[warp][lane] = incl - cnt;
-      pr_rec0[warp][lane] = r0;
-      pr_rec1[warp][lane] = r1;
-      __syncwarp();
-      // phase 3: cheap tests of each pair; passing pairs are compacted into
-      // tq and the contact math runs on full batches of 32
-      for (uint32_t eb = 0; eb < npairs; eb += 32u) {
-        const uint32_t e = eb + uint32_t(lane);
-        bool pass = false;
-        uint32_t ps = 0, pst = 0;
-        if (e < npairs) {
-          uint32_t lo = 0, hi = 31;  // owner: the last lane whose range starts at or before e
-          while (lo < hi) {
-            const uint32_t mid = (lo + hi + 1u) >> 1;
-            if (pr_ex[warp][mid] <= e) lo = mid; else hi = mid - 1u;
-          }
-          ps = pr_slot[warp][lo];
-          pst = pr_sb[warp][lo] + (e - pr_ex[warp][lo]);
-          pass = vt_entry<false>(s, c, th, ps, pst, pr_rec0[warp][lo], pr_rec1[warp][lo]);
-          if (pass && s.rec_vt) {
-            const uint2 tv = s.star_idx[pst];
-            record_vt(s, index, __float_as_uint(pr_rec1[warp][lo].w), tv.x, tv.y);
-          }
-        }
+    if (vqn >= 4u || (drain && vqn && !qn)) {  // 3: 4 pairs x 8 star entries a round
+      do {
+        const uint32_t nb = min(vqn, 4u), g = lane >> 3, ei = lane & 7u;
+        const uint32_t w = vqn - nb + min(g, nb - 1u);
+        const uint4 e = m.vq[w];
+        const uint32_t sn = g < nb ? e.z : 0u;
+        const uint32_t st = e.y + ei;
+        const bool pass = ei < sn && vt_box(s, m, e.x >> kScSlotBits, __uint_as_float(e.w), st);
         const uint32_t b = __ballot_sync(0xffffffffu, pass);
-        if (pass) {
-          const uint32_t kq = tqn + __popc(b & lt_mask);
-          tq_slot[warp][kq] = ps;
-          tq_st[warp][kq] = pst;
-        }
-        tqn += __popc(b);
-        __syncwarp();
-        if (tqn >= 32u) {
-          vt_entry<true>(s, c, th, tq_slot[warp][lane], tq_st[warp][lane]);
+        if (pass) m.bq[bqn + __popc(b & lt_mask)] = make_uint2(e.x, st);
+        bqn += __popc(b);
+        // a star of more than 8 entries keeps its pair queued with the rest
+        // of its range; the others' entries are used up
+        if (!__any_sync(0xffffffffu, sn > 8u)) {
+          vqn -= nb;
+        } else {
           __syncwarp();
-          tqn -= 32u;
-          if (uint32_t(lane) < tqn) {
-            tq_slot[warp][lane] = tq_slot[warp][32 + lane];
-            tq_st[warp][lane] = tq_st[warp][32 + lane];
-          }
+          if (ei == 0 && g < nb) m.vq[w] = make_uint4(e.x, e.y + 8u, sn > 8u ? sn - 8u : 0u, e.w);
           __syncwarp();
         }
+      } while (bqn < 32u && vqn >= 4u);
+      continue;
+    }
+    if (qn >= 32u || (drain && qn)) {  // 2
+      const uint32_t nb = min(qn, 32u);
+      qn -= nb;
+      uint32_t e = 0, sb = 0, sn = 0;
+      float eth = 0.f;
+      bool vv = false, vt = false;
+      if (lane < nb) {
+        e = m.q[qn + lane];
+        vt = sc_gate(s, m, e >> kScSlotBits, e & kScSlotMask, vv, sb, sn, eth);
+      }
+      const uint32_t bv = __ballot_sync(0xffffffffu, vv), b = __ballot_sync(0xffffffffu, vt);
+      if (vv) m.vv[vvn + __popc(bv & lt_mask)] = e;
+      vvn += __popc(bv);
+      if (vt) m.vq[vqn + __popc(b & lt_mask)] = make_uint4(e, sb, sn, __float_as_uint(eth));
+      vqn += __popc(b);
+      continue;
+    }
+    if (uqn >= 32u || (drain && uqn)) {
+      const uint32_t nb = min(uqn, 32u);
+      uqn -= nb;
+      if (lane < nb) {
+        const uint32_t e = m.uq[uqn + lane];
+        const unsigned long long key = sc_untangle_key(s, m, e >> kScSlotBits, e & kScSlotMask);
+        if (key != ~0ull) atomicMin(&m.best[e >> kScSlotBits], key);
       }
       __syncwarp();
+      if (best_in > 0.f) best_in = fminf(best_in, __uint_as_float(min(uint32_t(m.best[v] >> 32), 0x60AD78ECu)));
+      continue;
     }
+    if (drain) break;
+    if (cn >= kSub || (cn && pos >= total)) {  // 1: the staged candidates against the cluster
+      do {
+        const uint32_t nb = min(cn, kSub);
+        cn -= nb;
+        const uint32_t c = cn + min(sub, nb - 1u);
+        const bool on = mine && sub < nb;
+        const float4 a = m.cp[c];
+        const V3 d = pi - mk(a);
+        const float d2 = dot(d, d), r = reach + a.w;
+        const bool pass = on && d2 <= r * r;
+        const uint32_t b = __ballot_sync(0xffffffffu, pass);
+        const uint32_t e = v << kScSlotBits | m.cslot[c];
+        if (pass) m.q[qn + __popc(b & lt_mask)] = e;
+        qn += __popc(b);
+        if (max_layer) {
+          const bool track = on && m.clayer[c] < layer && d2 <= best_in;
+          const uint32_t bt = __ballot_sync(0xffffffffu, track);
+          if (track) m.uq[uqn + __popc(bt & lt_mask)] = e;
+          uqn += __popc(bt);
+        }
+      } while (cn >= kSub && qn < 32u && uqn < 32u);
+      continue;
+    }
+    if (pos < total) {  // stage candidates that come near the cluster
+      {
+        const uint32_t t = pos + lane;
+        pos += 32u;
+        bool keep = false;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+        uint32_t slot = 0, cl = 0;
+        if (t < total) {
+          while (t >= m.end[k]) ++k;
+          slot = m.beg[k] + t;
+          const float4 p = s.vs_p[slot], q = s.vs_q[slot];
+          cl = __float_as_uint(q.y);
+          a = make_float4(p.x, p.y, p.z, sc_reach(p.w, 1.3f * q.x, q.w));
+          const float r = blo.w + fmaxf(a.w, max_layer ? sc_reach(2.5f * p.w, 1.3f * q.x, 0.f) : 0.f);
+          const V3 d = mk(fmaxf(fmaxf(blo.x - p.x, p.x - bhi.x), 0.f), fmaxf(fmaxf(blo.y - p.y, p.y - bhi.y), 0.f),
+                          fmaxf(fmaxf(blo.z - p.z, p.z - bhi.z), 0.f));
+          keep = dot(d, d) <= r * r && ub.at(s.vs_c[slot]) == uint32_t(m.box[k]);
+        }
+        const uint32_t b = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+          const uint32_t q = cn + __popc(b & lt_mask);
+          m.cp[q] = a;
+          m.clayer[q] = cl;
+          m.cslot[q] = slot;
+        }
+        cn += __popc(b);
+      }
+      continue;
+    }
+    if (!todo) {
+      drain = true;
+      continue;
+    }
+    ub = union_box<kScV>(cell, todo, v, lane, mine);
+    todo &= ~__ballot_sync(0xffffffffu, mine);
+    total = union_ranges(ub, s.table, s.cs, m.end, m.beg, m.box, lane, [](uint32_t beg, uint32_t) { return beg; });
+    // the box around the vertices, and in blo.w the largest reach among them
+    // (an untangle candidate, within eth * 2.5 + 1.3 llj, included)
+    const float inf = __int_as_float(0x7F800000);
+    blo = mine ? make_float4(pi.x, pi.y, pi.z, best_in > 0.f ? fmaxf(reach, treach) : reach)
+               : make_float4(inf, inf, inf, 0.f);
+    bhi = mine ? pi : mk(-inf, -inf, -inf);
+    for (int o = 1; o < int(kScV); o <<= 1) {
+      blo.x = fminf(blo.x, __shfl_xor_sync(0xffffffffu, blo.x, o));
+      blo.y = fminf(blo.y, __shfl_xor_sync(0xffffffffu, blo.y, o));
+      blo.z = fminf(blo.z, __shfl_xor_sync(0xffffffffu, blo.z, o));
+      blo.w = fmaxf(blo.w, __shfl_xor_sync(0xffffffffu, blo.w, o));
+      bhi = vmax(bhi, mk(__shfl_xor_sync(0xffffffffu, bhi.x, o), __shfl_xor_sync(0xffffffffu, bhi.y, o),
+                         __shfl_xor_sync(0xffffffffu, bhi.z, o)));
+    }
+    pos = cn = k = 0;
   }
-  if (uint32_t(lane) < tqn) vt_entry<true>(s, c, th, tq_slot[warp][lane], tq_st[warp][lane]);
-  if (c.track) {
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best_in, o);
-      const uint32_t ot = __shfl_xor_sync(0xffffffffu, best_t, o);
-      const uint32_t oj = __shfl_xor_sync(0xffffffffu, best_j, o);
-      if (ob < best_in || (ob == best_in && ot < best_t)) { best_in = ob; best_t = ot; best_j = oj; }
+  if (best_in >= 0.f && live && sub == 0u) {
+    const unsigned long long key = m.best[v];
+    if (key != ~0ull) {
+      const uint32_t j = (uint32_t)s.vs_c[uint32_t(key) & kScSlotMask].w;
+      if (j < 0x3FFFFEu) s.acc[(size_t)index * A_N + A_UT] = (int32_t)(j + 1u);
     }
-    if (lane == 0 && best_j < 0x3FFFFEu) s.acc[(size_t)index * A_N + A_UT] = (int32_t)(best_j + 1u);
   }
 }
 
@@ -1420,34 +1675,21 @@ __global__ void __launch_bounds__(256, 3) k_ee_ccd(SCArgs s) {
     ee_listed_pair(s, s.ccd_q[q], false);
 }
 
-// One warp per edge; candidates of the 27 cells around the edge midpoint are
-// flattened in the reference's order (dz outer, dx inner) and visited 32 per
-// round.  The per-edge cap on counted candidates (search_count >
+// One edge, searched by a warp in the reference's order: candidates of the 27
+// cells around the edge midpoint are flattened (dz outer, dx inner) and visited
+// 32 per round.  The per-edge cap on counted candidates (search_count >
 // max_search_iterations, :356-359) is applied with a ballot prefix count, so
-// exactly the reference's first max_search counted pairs are processed.
-// kList: the counted pairs are appended to the pair list for k_ee_pairs
-// (the two-hop lists are then not staged here); otherwise the warp does
-// their contact work itself.
-// (__grid_constant__: the overflow call takes the arguments' address without
-// a per-thread copy.)  The filter alone is latency-bound and needs few
-// registers, so list mode asks for 8 blocks (64 warps) per SM.
-template <bool kList>
-__global__ void __launch_bounds__(256, kList ? 8 : 4) k_ee(const __grid_constant__ SCArgs s) {
-  __shared__ uint32_t sh_start[8][28], sh_end[8][28], sh_beg[8][28];
-  __shared__ uint32_t sh_th[8][2][kTwoHopCache];
-  __shared__ float sh_thr[8][2][kTwoHopCache];
-  __shared__ uint32_t sh_q[8][32 * kRounds];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t ei = blockIdx.x * 8u + warp;
-  if (ei >= s.ne) return;  // whole warp
-  const EdgeCtx c = edge_ctx(s, ei);
-  const int4 bc4 = s.ecell[ei];
+// exactly the reference's first max_search counted pairs are taken.
+struct EeSearch {
+  uint32_t start[28], end[28], beg[28];
+  uint32_t q[32 * kRounds];
+};
+// the counted pairs of up to 32 * kRounds candidates at a time go to
+// take(queue of candidate slots, length)
+template <class F>
+__device__ __forceinline__ void ee_search(const SCArgs& s, const EdgeCtx& c, EeSearch& m, int lane, F&& take) {
+  const int4 bc4 = s.ecell[c.ei];
   const I3 base = I3{bc4.x, bc4.y, bc4.z};
-  TwoHop th0{}, th1{};
-  if (!kList) {
-    th0 = stage_two_hop(s.th_off, s.th_idx, s.th_rest, c.u0, sh_th[warp][0], sh_thr[warp][0], lane);
-    th1 = stage_two_hop(s.th_off, s.th_idx, s.th_rest, c.u1, sh_th[warp][1], sh_thr[warp][1], lane);
-  }
   // lane k = (dz+1)*9 + (dy+1)*3 + (dx+1)
   uint32_t cnt = 0, beg = 0;
   if (lane < 27) {
@@ -1459,7 +1701,7 @@ __global__ void __launch_bounds__(256, kList ? 8 : 4) k_ee(const __grid_constant
     uint32_t lo = beg, hi = en > beg ? en : beg;
     while (lo < hi) {
       const uint32_t mid = lo + (hi - lo) / 2u;
-      if ((uint32_t)s.es_c[mid].w <= ei) lo = mid + 1u; else hi = mid;
+      if ((uint32_t)s.es_c[mid].w <= c.ei) lo = mid + 1u; else hi = mid;
     }
     beg = lo;
     cnt = en > beg ? en - beg : 0u;
@@ -1469,77 +1711,261 @@ __global__ void __launch_bounds__(256, kList ? 8 : 4) k_ee(const __grid_constant
     const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += v;
   }
+  __syncwarp();
   if (lane < 27) {
-    sh_start[warp][lane] = incl - cnt;
-    sh_end[warp][lane] = incl;
-    sh_beg[warp][lane] = beg;
+    m.start[lane] = incl - cnt;
+    m.end[lane] = incl;
+    m.beg[lane] = beg;
   }
   __syncwarp();
   const uint32_t total = __shfl_sync(0xffffffffu, incl, 26);
   uint32_t counted = 0;
   int k = 0;
-  uint32_t* queue = sh_q[warp];
   const uint32_t lt_mask = (1u << lane) - 1u;
   for (uint32_t chunk = 0; chunk < total && counted < s.max_search; chunk += 32u * kRounds) {
-    // phase 1: counting filter; the first max_search counted pairs are queued
     uint32_t qn = 0;
     for (uint32_t r = 0; r < kRounds; ++r) {
       const uint32_t t = chunk + r * 32u + lane;
       bool pass = false;
-      uint32_t slot = 0, eb_l = 0;
+      uint32_t slot = 0;
       if (t < total) {
-        while (t >= sh_end[warp][k]) ++k;
-        slot = sh_beg[warp][k] + (t - sh_start[warp][k]);
+        while (t >= m.end[k]) ++k;
+        slot = m.beg[k] + (t - m.start[k]);
         // one level of loads for the whole filter
         const int4 bc = s.es_c[slot];
         const float4 bmin = s.es_lo[slot], bmax = s.es_hi[slot];
         const uint2 ebv = make_uint2(__float_as_uint(bmin.w), __float_as_uint(bmax.w));
         const uint32_t eb = (uint32_t)bc.w;
-        eb_l = eb;
-        pass = ei < eb && !(ebv.x == c.u0 || ebv.x == c.u1 || ebv.y == c.u0 || ebv.y == c.u1) &&
+        pass = c.ei < eb && !(ebv.x == c.u0 || ebv.x == c.u1 || ebv.y == c.u0 || ebv.y == c.u1) &&
                bc.x == base.x - 1 + k % 3 && bc.y == base.y - 1 + (k / 3) % 3 && bc.z == base.z - 1 + k / 9 &&
                !(c.amin.x > bmax.x || c.amin.y > bmax.y || c.amin.z > bmax.z || c.amax.x < bmin.x ||
                  c.amax.y < bmin.y || c.amax.z < bmin.z);
       }
       const uint32_t b = __ballot_sync(0xffffffffu, pass);
       const uint32_t rank = counted + __popc(b & lt_mask);
-      // list mode queues the edge index, otherwise the slot of its records
-      if (pass && rank < s.max_search) queue[qn + __popc(b & lt_mask)] = kList ? eb_l : slot;
+      if (pass && rank < s.max_search) m.q[qn + __popc(b & lt_mask)] = slot;
       const uint32_t nb = __popc(b);
       qn += counted + nb <= s.max_search ? nb : (counted < s.max_search ? s.max_search - counted : 0u);
       counted += nb;
     }
     __syncwarp();
-    if constexpr (kList) {
-      // phase 2: the queued pairs are appended to this block's segment of
-      // the pair list of k_ee_pairs; those past its capacity get their
-      // contact work here
-      const uint32_t seg = blockIdx.x % kEeSeg, segcap = s.ee_cap / kEeSeg;
-      uint32_t lbase = segcap;
-      if (lane == 0 && qn && segcap) lbase = atomicAdd(s.ee_n + seg, qn);
-      lbase = __shfl_sync(0xffffffffu, lbase, 0);
-      for (uint32_t q = lane; q < qn; q += 32u) {
-        const uint32_t eb = queue[q];
-        if (lbase < segcap && q < segcap - lbase) {
-          s.ee_q[size_t(seg) * segcap + lbase + q] = make_uint2(ei, eb);
-        } else {
-          if (s.rec_ee) record_ee(s, ei, eb);
-          ee_listed_pair_call(s, make_uint2(ei, eb));
-        }
-      }
-    } else {
-      // phase 2: contact work on the queued pairs
-      for (uint32_t q = lane; q < qn; q += 32u) {
-        const uint32_t slot = queue[q];
-        const uint32_t eb = (uint32_t)s.es_c[slot].w;
-        const uint2 ebv = s.es_v[slot];
-        const float4 qj = s.p4[ebv.x], qvj = s.p4[ebv.y], xj = s.x4[ebv.x], xvj = s.x4[ebv.y];
-        if (s.rec_ee) record_ee(s, ei, eb);
-        ee_pair(s, c, th0, th1, eb, ebv.x, ebv.y, qj, qvj, xj, xvj, true);
-      }
-    }
+    take(m.q, qn);
     __syncwarp();
   }
+}
+
+// A warp appends qn pairs to its block's segment of the pair list of
+// k_ee_pairs; pairs past the segment's capacity get their contact work here.
+// pair(q): the q-th.
+template <class F>
+__device__ __forceinline__ void ee_append(const SCArgs& s, uint32_t qn, uint32_t lane, F&& pair) {
+  const uint32_t seg = blockIdx.x % kEeSeg, segcap = s.ee_cap / kEeSeg;
+  uint32_t lbase = segcap;
+  if (lane == 0 && qn && segcap) lbase = atomicAdd(s.ee_n + seg, qn);
+  lbase = __shfl_sync(0xffffffffu, lbase, 0);
+  for (uint32_t q = lane; q < qn; q += 32u) {
+    const uint2 pr = pair(q);
+    if (lbase < segcap && q < segcap - lbase) {
+      s.ee_q[size_t(seg) * segcap + lbase + q] = pr;
+    } else {
+      if (s.rec_ee) record_ee(s, pr.x, pr.y);
+      ee_listed_pair_call(s, pr);
+    }
+  }
+}
+__device__ __noinline__ void ee_list_ordered(const SCArgs& s, uint32_t ei, EeSearch& m, int lane) {
+  ee_search(s, edge_ctx(s, ei), m, lane, [&](const uint32_t* q, uint32_t qn) {
+    ee_append(s, qn, uint32_t(lane), [&](uint32_t i) { return make_uint2(ei, (uint32_t)s.es_c[q[i]].w); });
+  });
+}
+
+// Counted (edge, edge) pairs for k_ee_pairs.  As in k_sc_solve a warp works a
+// cluster of kEeV edges that are neighbours in space: the union of their
+// 27-cell neighbourhoods is staged 32 candidates at a time in shared memory,
+// those that miss the box around all of the cluster's swept boxes are dropped
+// there, and 32 / kEeV candidates are tested against all the edges at once.  Counted
+// pairs wait in shared memory until the cluster's search is over; an edge with
+// more than max_search of them is searched again in the reference's order
+// (ee_list_ordered), as is every edge of a cluster whose pairs outgrow the
+// buffer.  The list's order is free.  A warp per edge (candidates over the
+// lanes) took 0.45 ms per pass on config 2 (391,682 edges, 13.6 counted pairs
+// each), most of it bucket walks and searches.
+constexpr int kEeClusterWarps = 4;
+constexpr uint32_t kEeV = 8;         // edges per warp
+constexpr uint32_t kEePairBuf = 288;
+constexpr uint32_t kEeEdgeBits = 29;  // buffered pairs: edge of the cluster << 29 | candidate edge
+struct EeWarp {
+  uint32_t end[kScCells], beg[kScCells];  // (see ScWarp)
+  uint8_t box[kScCells];
+  float4 lo[36], hi[36];  // staged candidates: swept box, endpoints in .w
+  uint2 c[36];            // cell in the box (x, y, z bytes), index
+  uint32_t edge[kEeV];
+  union {
+    uint32_t pq[kEePairBuf];
+    EeSearch search;
+  };
+};
+__global__ void __launch_bounds__(32 * kEeClusterWarps, 8) k_ee_cluster(const __grid_constant__ SCArgs s) {
+  __shared__ EeWarp sh[kEeClusterWarps];
+  const uint32_t lane = threadIdx.x & 31u;
+  EeWarp& m = sh[threadIdx.x >> 5];
+  const uint32_t lt_mask = (1u << lane) - 1u;
+  const uint32_t at = (blockIdx.x * kEeClusterWarps + (threadIdx.x >> 5)) * kEeV;
+  if (at >= s.ne) return;  // whole warp
+  const uint32_t v = lane % kEeV, sub = lane / kEeV;
+  constexpr uint32_t kSub = 32u / kEeV;
+  const bool live = at + v < s.ne;
+  uint32_t ei = 0xFFFFFFFFu, u0 = 0, u1 = 0, vmask = 0;
+  V3 amin = mk(0.f, 0.f, 0.f), amax = amin;
+  I3 cell{0, 0, 0};
+  for (uint32_t q = v; q < 32u; q += kEeV) vmask |= 1u << q;
+  if (live) {
+    ei = s.eorder[at + v];
+    const EdgeCtx c = edge_ctx(s, ei);
+    u0 = c.u0;
+    u1 = c.u1;
+    amin = c.amin;
+    amax = c.amax;
+    const int4 bc = s.ecell[ei];
+    cell = I3{bc.x, bc.y, bc.z};
+    m.edge[v] = ei;
+  }
+  uint32_t todo = __ballot_sync(0xffffffffu, live);
+  while (todo) {
+    bool mine;
+    const UnionBox ub = union_box<kEeV>(cell, todo, v, lane, mine);
+    todo &= ~__ballot_sync(0xffffffffu, mine);
+    const uint32_t first = __reduce_min_sync(0xffffffffu, mine ? ei : 0xFFFFFFFFu);
+    // buckets are in ascending edge order and a pair belongs to its smaller
+    // edge index: start past the cluster's smallest
+    const uint32_t total = union_ranges(ub, s.table, s.ecs, m.end, m.beg, m.box, lane, [&](uint32_t beg, uint32_t en) {
+      uint32_t lo = beg;
+      while (lo < en) {
+        const uint32_t mid = lo + (en - lo) / 2u;
+        if ((uint32_t)s.es_c[mid].w <= first) lo = mid + 1u; else en = mid;
+      }
+      return lo;
+    });
+    const uint32_t rx = uint32_t(cell.x - ub.ox) - 1u, ry = uint32_t(cell.y - ub.oy) - 1u,
+                   rz = uint32_t(cell.z - ub.oz) - 1u;
+    // the box around the edges' swept boxes; unbounded with a NaN among them,
+    // whose box test rejects nothing
+    const bool odd = mine && !(amin.x <= amax.x && amin.y <= amax.y && amin.z <= amax.z);
+    const float inf = __any_sync(0xffffffffu, odd) ? -__int_as_float(0x7F800000) : __int_as_float(0x7F800000);
+    V3 blo = mine && !odd ? vmin(amin, mk(inf, inf, inf)) : mk(inf, inf, inf);
+    V3 bhi = mine && !odd ? vmax(amax, mk(-inf, -inf, -inf)) : mk(-inf, -inf, -inf);
+    for (int o = 1; o < int(kEeV); o <<= 1) {
+      blo = vmin(blo, mk(__shfl_xor_sync(0xffffffffu, blo.x, o), __shfl_xor_sync(0xffffffffu, blo.y, o),
+                         __shfl_xor_sync(0xffffffffu, blo.z, o)));
+      bhi = vmax(bhi, mk(__shfl_xor_sync(0xffffffffu, bhi.x, o), __shfl_xor_sync(0xffffffffu, bhi.y, o),
+                         __shfl_xor_sync(0xffffffffu, bhi.z, o)));
+    }
+    uint32_t counted = 0, pn = 0, k = 0, cn = 0;
+    bool full = false;
+    for (uint32_t pos = 0; pos < total && !full; pos += 32u) {
+      const uint32_t t = pos + lane;
+      bool keep = false;
+      float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+      int4 c = make_int4(0, 0, 0, 0);
+      if (t < total) {
+        while (t >= m.end[k]) ++k;
+        const uint32_t slot = m.beg[k] + t;
+        c = s.es_c[slot];
+        lo = s.es_lo[slot];
+        hi = s.es_hi[slot];
+        keep = ub.at(c) == uint32_t(m.box[k]) && !(blo.x > hi.x || blo.y > hi.y || blo.z > hi.z || bhi.x < lo.x ||
+                                                   bhi.y < lo.y || bhi.z < lo.z);
+      }
+      const uint32_t kb = __ballot_sync(0xffffffffu, keep);
+      if (keep) {
+        const uint32_t q = cn + __popc(kb & lt_mask);
+        m.lo[q] = lo;
+        m.hi[q] = hi;
+        m.c[q] = make_uint2(uint32_t(c.x - ub.ox) | uint32_t(c.y - ub.oy) << 8 | uint32_t(c.z - ub.oz) << 16, uint32_t(c.w));
+      }
+      cn += __popc(kb);
+      __syncwarp();
+      // kSub at a time from the end; fewer than that wait for the next round
+      const bool last = pos + 32u >= total;
+      while (cn >= kSub || (last && cn)) {
+        const uint32_t nb = min(cn, kSub);
+        cn -= nb;
+        const uint32_t ci = cn + sub;
+        bool pass = false;
+        uint32_t eb = 0;
+        if (mine && sub < nb) {
+          const float4 clo = m.lo[ci], chi = m.hi[ci];
+          if (!(amin.x > chi.x || amin.y > chi.y || amin.z > chi.z || amax.x < clo.x || amax.y < clo.y ||
+                amax.z < clo.z)) {
+            const uint2 bc = m.c[ci];
+            const uint32_t b0 = __float_as_uint(clo.w), b1 = __float_as_uint(chi.w);
+            eb = bc.y;
+            // (cells apart by at most 1 on each axis: 0, 1 or 2 from the edge's cell - 1)
+            pass = ei < eb && !(b0 == u0 || b0 == u1 || b1 == u0 || b1 == u1) && (bc.x & 0xFFu) - rx <= 2u &&
+                   ((bc.x >> 8) & 0xFFu) - ry <= 2u && (bc.x >> 16) - rz <= 2u;
+          }
+        }
+        const uint32_t b = __ballot_sync(0xffffffffu, pass);
+        if (pass) m.pq[pn + __popc(b & lt_mask)] = v << kEeEdgeBits | eb;
+        pn += __popc(b);
+        counted += __popc(b & vmask);
+        if (pn > kEePairBuf - 32u) {
+          full = true;
+          break;
+        }
+      }
+      __syncwarp();
+    }
+    __syncwarp();
+    const bool again = mine && (full || counted > s.max_search);
+    const uint32_t over = __ballot_sync(0xffffffffu, again && sub == 0u);  // bit v
+    if (!full) {
+      uint32_t kept = pn;
+      if (over) {  // drop the pairs of the edges that are searched again
+        kept = 0;
+        for (uint32_t q0 = 0; q0 < pn; q0 += 32u) {
+          const uint32_t q = q0 + lane, e = q < pn ? m.pq[q] : 0u;
+          const bool keep = q < pn && !((over >> (e >> kEeEdgeBits)) & 1u);
+          const uint32_t b = __ballot_sync(0xffffffffu, keep);
+          if (keep) m.pq[kept + __popc(b & lt_mask)] = e;
+          kept += __popc(b);
+          __syncwarp();
+        }
+      }
+      ee_append(s, kept, lane, [&](uint32_t q) {
+        const uint32_t e = m.pq[q];
+        return make_uint2(m.edge[e >> kEeEdgeBits], e & ((1u << kEeEdgeBits) - 1u));
+      });
+      __syncwarp();  // the buffer is the ordered search's too
+    }
+    for (uint32_t o = over; o; o &= o - 1u)
+      ee_list_ordered(s, __shfl_sync(0xffffffffu, ei, __ffs(o) - 1), m.search, int(lane));
+    __syncwarp();
+  }
+}
+
+// The search with the contact work in the edge's warp: a warp per edge, no
+// pair list.
+__global__ void __launch_bounds__(256, 4) k_ee(const __grid_constant__ SCArgs s) {
+  __shared__ EeSearch sh[8];
+  __shared__ uint32_t sh_th[8][2][kTwoHopCache];
+  __shared__ float sh_thr[8][2][kTwoHopCache];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t ei = blockIdx.x * 8u + warp;
+  if (ei >= s.ne) return;  // whole warp
+  const EdgeCtx c = edge_ctx(s, ei);
+  const TwoHop th0 = stage_two_hop(s.th_off, s.th_idx, s.th_rest, c.u0, sh_th[warp][0], sh_thr[warp][0], lane);
+  const TwoHop th1 = stage_two_hop(s.th_off, s.th_idx, s.th_rest, c.u1, sh_th[warp][1], sh_thr[warp][1], lane);
+  ee_search(s, c, sh[warp], lane, [&](const uint32_t* queue, uint32_t qn) {
+    for (uint32_t q = lane; q < qn; q += 32u) {
+      const uint32_t slot = queue[q];
+      const uint32_t eb = (uint32_t)s.es_c[slot].w;
+      const uint2 ebv = s.es_v[slot];
+      const float4 qj = s.p4[ebv.x], qvj = s.p4[ebv.y], xj = s.x4[ebv.x], xvj = s.x4[ebv.y];
+      if (s.rec_ee) record_ee(s, ei, eb);
+      ee_pair(s, c, th0, th1, eb, ebv.x, ebv.y, qj, qvj, xj, xvj, true);
+    }
+  });
 }
 
 // Grouped variant of k_ee, one lane per edge.  A warp takes 32 consecutive

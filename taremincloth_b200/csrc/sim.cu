@@ -613,7 +613,8 @@ struct Sim {
   DBuf<float4> nrm;
   DBuf<int32_t> acc;
   DBuf<int4> vcell, ecell;
-  DBuf<float4> sbox;
+  DBuf<float4> sbox, st_lo, st_hi;
+  DBuf<float> st_mz;
   DBuf<float> mlen;
   DBuf<float4> eamin, eamax;
   DBuf<float4> vs_p, vs_q, es_lo, es_hi;
@@ -1026,6 +1027,26 @@ struct Sim {
     TC_CK(cudaStreamSynchronize(st));
   }
 
+  // Morton order of points, one scale for all axes (a flat cloth's small
+  // extent must not take part in the order on equal terms)
+  template <class F>
+  static std::vector<uint32_t> space_order(uint32_t cnt, F&& at) {
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (uint32_t i = 0; i < cnt; ++i)
+      for (int k = 0; k < 3; ++k) {
+        lo[k] = std::fmin(lo[k], at(i, k));
+        hi[k] = std::fmax(hi[k], at(i, k));
+      }
+    const float ext = std::fmax(hi[0] - lo[0], std::fmax(hi[1] - lo[1], hi[2] - lo[2]));
+    const float sc = ext > 0.f ? 1.f / ext : 0.f, inv[3] = {sc, sc, sc};
+    std::vector<uint64_t> key(cnt);
+    for (uint32_t i = 0; i < cnt; ++i)
+      key[i] = uint64_t(tcloth::morton3(at(i, 0), at(i, 1), at(i, 2), lo, inv)) << 32 | i;
+    std::sort(key.begin(), key.end());
+    std::vector<uint32_t> ord(cnt);
+    for (uint32_t i = 0; i < cnt; ++i) ord[i] = uint32_t(key[i]);
+    return ord;
+  }
   void init(const MeshInput& in, int dev) {
     device = dev;
     TC_CK(cudaSetDevice(device));
@@ -1035,25 +1056,14 @@ struct Sim {
     m = build_mesh(in);
     cell_ref = m.cell;
     n = m.n;
-    {  // vertices of one warp close in space for the collider pass (any order is exact)
-      float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-      for (uint32_t i = 0; i < n; ++i)
-        for (int k = 0; k < 3; ++k) {
-          lo[k] = std::fmin(lo[k], m.pos[3 * size_t(i) + k]);
-          hi[k] = std::fmax(hi[k], m.pos[3 * size_t(i) + k]);
-        }
-      float inv[3];
-      for (int k = 0; k < 3; ++k) inv[k] = hi[k] > lo[k] ? 1.f / (hi[k] - lo[k]) : 0.f;
-      std::vector<std::pair<uint32_t, uint32_t>> code(n);
-      for (uint32_t i = 0; i < n; ++i)
-        code[i] = {tcloth::morton3(m.pos[3 * size_t(i)], m.pos[3 * size_t(i) + 1], m.pos[3 * size_t(i) + 2], lo, inv),
-                   i};
-      std::sort(code.begin(), code.end());
-      std::vector<uint32_t> ord(n);
-      for (uint32_t i = 0; i < n; ++i) ord[i] = code[i].second;
-      col_order.upload(ord, st);
-      col_order_h = std::move(ord);
-    }
+    // vertices and edges of one warp close in space, for the passes that may
+    // work them in any order
+    col_order_h = space_order(n, [&](uint32_t i, int k) { return m.pos[3 * size_t(i) + k]; });
+    col_order.upload(col_order_h, st);
+    edge_order.upload(space_order(uint32_t(m.edges.size() / 2), [&](uint32_t e, int k) {
+      return 0.5f * (m.pos[3 * size_t(m.edges[2 * size_t(e)]) + k] + m.pos[3 * size_t(m.edges[2 * size_t(e) + 1]) + k]);
+    }), st);
+    TC_CK(cudaStreamSynchronize(st));
     nd = uint32_t(m.dist.size());
     nb = uint32_t(m.bend.size());
     ne = uint32_t(m.edges.size() / 2);
@@ -1121,7 +1131,9 @@ struct Sim {
     TC_CK(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
     nrm.alloc(n);
     acc.alloc(size_t(n) * A_N);
-    vcell.alloc(n); mlen.alloc(n); sbox.alloc(3 * size_t(n)); ecell.alloc(ne); eamin.alloc(ne); eamax.alloc(ne);
+    vcell.alloc(n); mlen.alloc(n); sbox.alloc(3 * size_t(n));
+    st_lo.alloc(m.star_idx.size() / 2); st_hi.alloc(m.star_idx.size() / 2); st_mz.alloc(m.star_idx.size() / 2);
+    ecell.alloc(ne); eamin.alloc(ne); eamax.alloc(ne);
     ccd_q.alloc(size_t(ne) * 8 + 1024); ccd_n.alloc(1 + tcloth::kEeSeg);
     ee_q.alloc(size_t(ne) * 24 + 1024);
     vs_p.alloc(n); vs_q.alloc(n); vs_c.alloc(n); tile_sum.alloc(64); es_c.alloc(ne); es_v.alloc(ne); es_lo.alloc(ne); es_hi.alloc(ne);
@@ -1326,7 +1338,8 @@ struct Sim {
     a.adj_off = adj_off.p; a.adj_idx = adj_idx.p; a.th_off = th_off.p; a.th_idx = th_idx.p; a.th_rest = th_rest.p;
     a.star_off = star_off.p; a.star_idx = star_idx.p; a.edges = edges.p; a.edge_bits = edge_bits.p;
     a.cs = cs.p; a.srt = srt.p; a.ecs = ecs.p; a.esrt = esrt.p; a.nrm = nrm.p; a.acc = acc.p;
-    a.sbox = sbox.p;
+    a.sbox = sbox.p; a.st_lo = st_lo.p; a.st_hi = st_hi.p; a.st_mz = st_mz.p;
+    a.order = col_order.p; a.eorder = edge_order.p;
     a.vcell = vcell.p; a.mlen = mlen.p; a.ecell = ecell.p; a.eamin = eamin.p; a.eamax = eamax.p;
     a.ccd_q = ccd_q.p; a.ccd_n = ccd_n.p; a.ccd_cap = uint32_t(ccd_q.n);
     a.ee_q = ee_q.p; a.ee_n = ccd_n.p ? ccd_n.p + 1 : nullptr;
@@ -1344,7 +1357,7 @@ struct Sim {
   // results do not depend on it)
   uint32_t col_block = 256;
   // the collider pass's vertex order: Morton order of the initial positions
-  DBuf<uint32_t> col_order;
+  DBuf<uint32_t> col_order, edge_order;
   float cell_ref = 0.f;  // the reference formula's hash cell (tc_set_hash_cell_size can override m.cell)
   // E-E kernel: false = one warp per edge (k_ee), true = one lane per edge
   // with per-cell candidate lists in shared memory (k_ee_grouped); same pairs
@@ -1402,8 +1415,9 @@ struct Sim {
       if (ee_grouped) {
         k_ee_grouped<<<grid(ne, 32 * tcloth::kEeWarps), 32 * tcloth::kEeWarps, 0, ss>>>(a);
       } else {
-        if (a.ee_cap) k_ee<true><<<grid(ne, 8), 256, 0, ss>>>(a);
-        else k_ee<false><<<grid(ne, 8), 256, 0, ss>>>(a);
+        if (a.ee_cap)
+          k_ee_cluster<<<grid(ne, tcloth::kEeV * tcloth::kEeClusterWarps), 32 * tcloth::kEeClusterWarps, 0, ss>>>(a);
+        else k_ee<<<grid(ne, 8), 256, 0, ss>>>(a);
         if (a.ee_cap) k_ee_pairs<<<tcloth::kEeSeg * tcloth::kEePairBlocks, 256, 0, ss>>>(a);
       }
     });
@@ -1477,9 +1491,9 @@ struct Sim {
       TC_CK(cudaEventRecord(ev_join, st2));
     }
     encode_hash(0);
-    timed("sc_star_box", [&] { k_star_box<<<grid(n, 256), 256, 0, st>>>(n, star_off.p, star_idx.p, x4.p, p4.p, sbox.p); });
+    timed("sc_star_box", [&] { k_star_box<<<grid(n, 256), 256, 0, st>>>(n, star_off.p, star_idx.p, x4.p, p4.p, sbox.p, st_lo.p, st_hi.p, st_mz.p); });
     if (edges_on && !fork) encode_hash(1);
-    timed("sc_solve", [&] { k_sc_solve<<<grid(n, 8), 256, 0, st>>>(a); });
+    timed("sc_solve", [&] { k_sc_solve<<<grid(n, tcloth::kScV * tcloth::kScWarps), 32 * tcloth::kScWarps, 0, st>>>(a); });
     if (a.untangle) timed("sc_untangle", [&] { k_untangle<<<grid(n, 128), 128, 0, st>>>(a); });
     if (fork) TC_CK(cudaStreamWaitEvent(st, ev_join, 0));
     if (edges_on && !fork) encode_ee(a, st);

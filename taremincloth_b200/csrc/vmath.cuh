@@ -47,7 +47,7 @@ constexpr float kEps = 1e-7f;
 // hash_coords (shaders/spatial_grid_sort.wgsl:25-31)
 __device__ __forceinline__ uint32_t hash3(int32_t cx, int32_t cy, int32_t cz, uint32_t table) {
   uint32_t h = ((uint32_t)cx * 73856093u) ^ ((uint32_t)cy * 19349663u) ^ ((uint32_t)cz * 83492791u);
-  return h % table;
+  return (table & (table - 1u)) == 0u ? h & (table - 1u) : h % table;  // the built tables are powers of two
 }
 struct I3 {
   int32_t x, y, z;
