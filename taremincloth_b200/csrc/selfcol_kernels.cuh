@@ -486,7 +486,7 @@ __device__ __forceinline__ bool near_folded_sq(const SCArgs& s, uint32_t a, uint
 }
 
 // ---------------- sc_solve: shaders/self_collision.wgsl:317-681
-// A warp works a cluster of kScV vertices that are neighbours in space.  Their
+// A warp works a cluster of kScV (1 to 8) vertices that are neighbours in space.  Their
 // 27-cell neighbourhoods overlap, so the union of the buckets is scanned once:
 // the candidates are staged in shared memory, 32 / kScV of them are tested
 // against all the vertices at a time, a shared load and a dozen operations for
@@ -508,9 +508,10 @@ __device__ __forceinline__ bool near_folded_sq(const SCArgs& s, uint32_t a, uint
 // first-strict-minimum scan in its visiting order (cx outer, cz inner, bucket
 // order inside a cell), is the minimum of (distance^2, that order).
 //
-// A warp per vertex (candidates over the lanes) spent 6,500 warp instructions
-// a vertex, most of them on bucket walks, compaction and batches of a few
-// lanes: 1.20 ms per pass on config 2.
+// A warp per vertex with its own bucket walk, compaction and batches of a few
+// lanes spent 6,500 warp instructions a vertex: 1.20 ms per pass on config 2,
+// now 3,250 and 0.79 ms, bound by instruction issue and the latency of the
+// gathers (7 blocks of 4 warps per SM; 8 spill, 6 leave latency uncovered).
 struct VertCtx {
   uint32_t index;
   bool pin_i;
@@ -519,10 +520,10 @@ struct VertCtx {
   I3 cell;
 };
 constexpr int kScWarps = 4;            // warps per block
-constexpr uint32_t kScV = 8;           // vertices per warp
 constexpr uint32_t kScCells = 96;      // cells of a union
 constexpr uint32_t kScSlotBits = 27;   // queue entries: vertex << 27 | slot
 constexpr uint32_t kScSlotMask = (1u << kScSlotBits) - 1u;
+template <uint32_t kScV>
 struct ScWarp {
   // the cluster's vertices
   uint32_t index[kScV], pin[kScV], th_b[kScV], th_n[kScV], th_first[kScV], th_last[kScV];
@@ -533,8 +534,8 @@ struct ScWarp {
   uint32_t end[kScCells], beg[kScCells];
   uint8_t box[kScCells];
   // staged candidates: p and reach, layer, slot
-  float4 cp[36];
-  uint32_t clayer[36], cslot[36];
+  float4 cp[32u + 32u / kScV];
+  uint32_t clayer[32u + 32u / kScV], cslot[32u + 32u / kScV];
   uint32_t q[64];                       // past the scan
   uint32_t uq[64];                      // untangle candidates past the scan
   uint4 vq[36];                         // past the gate: pair, star range, contact thickness
@@ -547,7 +548,8 @@ struct ScWarp {
   }
 };
 // two-hop list of the cluster's vertex i (see th_find)
-__device__ __forceinline__ bool sc_th_find(const SCArgs& s, const ScWarp& m, uint32_t i, uint32_t b, uint32_t& pos) {
+template <class W>
+__device__ __forceinline__ bool sc_th_find(const SCArgs& s, const W& m, uint32_t i, uint32_t b, uint32_t& pos) {
   // most vertices met in contact belong to another part of the mesh
   if (b < m.th_first[i] || b > m.th_last[i]) return false;
   uint32_t at = m.th_b[i];
@@ -559,7 +561,8 @@ __device__ __forceinline__ bool sc_th_find(const SCArgs& s, const ScWarp& m, uin
   pos = at;
   return s.th_idx[at] == b;
 }
-__device__ __forceinline__ bool sc_within2(const SCArgs& s, const ScWarp& m, uint32_t i, uint32_t b) {
+template <class W>
+__device__ __forceinline__ bool sc_within2(const SCArgs& s, const W& m, uint32_t i, uint32_t b) {
   uint32_t q;
   return m.index[i] == b || sc_th_find(s, m, i, b, q);
 }
@@ -673,7 +676,8 @@ __device__ __forceinline__ float sc_reach(float th, float ll_part, float ml) {
 // vertex i, candidate slot.  vv: the vertex-vertex contact math must run
 // (vv_contact); true with the star range of the candidate and the contact
 // thickness when its incident triangles must be tested.
-__device__ __forceinline__ bool sc_gate(const SCArgs& s, const ScWarp& m, uint32_t i, uint32_t slot, bool& vv,
+template <class W>
+__device__ __forceinline__ bool sc_gate(const SCArgs& s, const W& m, uint32_t i, uint32_t slot, bool& vv,
                                         uint32_t& st_b, uint32_t& st_n, float& out_eth) {
   vv = false;
   const VertCtx c = m.ctx(i);
@@ -721,7 +725,8 @@ __device__ __forceinline__ bool sc_gate(const SCArgs& s, const ScWarp& m, uint32
 }
 // One untangle candidate of the cluster's vertex i (:377-383): its key
 // (distance^2 bits, visiting order), or all ones.
-__device__ __forceinline__ unsigned long long sc_untangle_key(const SCArgs& s, const ScWarp& m, uint32_t i,
+template <class W>
+__device__ __forceinline__ unsigned long long sc_untangle_key(const SCArgs& s, const W& m, uint32_t i,
                                                               uint32_t slot) {
   const int4 jc = s.vs_c[slot];
   const float4 pj4 = s.vs_p[slot];
@@ -813,7 +818,8 @@ __device__ __forceinline__ void vv_contact(const SCArgs& s, uint32_t index, uint
 //
 // vt_box: the swept box of the vertex against the triangle's, on the star
 // entry's record and the contact thickness eth of (i, j)
-__device__ __forceinline__ bool vt_box(const SCArgs& s, const ScWarp& m, uint32_t i, float eth, uint32_t st) {
+template <class W>
+__device__ __forceinline__ bool vt_box(const SCArgs& s, const W& m, uint32_t i, float eth, uint32_t st) {
   const float4 tlo = s.st_lo[st], thi = s.st_hi[st];
   const float mz = s.st_mz[st];
   const V3 pi = mk(m.px[i], m.py[i], m.pz[i]);
@@ -825,7 +831,8 @@ __device__ __forceinline__ bool vt_box(const SCArgs& s, const ScWarp& m, uint32_
 // ownership (:486-500): the triangle is tested from its in-range vertex of
 // smallest index, so only a vertex below j can take it away; then the two-hop
 // exclusion
-__device__ __forceinline__ bool vt_owner(const SCArgs& s, const ScWarp& m, uint32_t i, uint32_t j, uint32_t st) {
+template <class W>
+__device__ __forceinline__ bool vt_owner(const SCArgs& s, const W& m, uint32_t i, uint32_t j, uint32_t st) {
   const uint2 pr = s.star_idx[st];
   const uint32_t index = m.index[i];
   if (pr.x == index || pr.y == index) return false;
@@ -983,10 +990,11 @@ __device__ __forceinline__ void vt_contact(const SCArgs& s, bool on, uint32_t in
   }
 }
 
+template <uint32_t kScV>
 __global__ void __launch_bounds__(32 * kScWarps, 7) k_sc_solve(const __grid_constant__ SCArgs s) {
-  __shared__ ScWarp sh[kScWarps];
+  __shared__ ScWarp<kScV> sh[kScWarps];
   const uint32_t lane = threadIdx.x & 31u;
-  ScWarp& m = sh[threadIdx.x >> 5];
+  ScWarp<kScV>& m = sh[threadIdx.x >> 5];
   const uint32_t lt_mask = (1u << lane) - 1u;
   const uint32_t at = (blockIdx.x * kScWarps + (threadIdx.x >> 5)) * kScV;
   if (at >= s.n) return;  // whole warp
@@ -1791,24 +1799,25 @@ __device__ __noinline__ void ee_list_ordered(const SCArgs& s, uint32_t ei, EeSea
 // lanes) took 0.45 ms per pass on config 2 (391,682 edges, 13.6 counted pairs
 // each), most of it bucket walks and searches.
 constexpr int kEeClusterWarps = 4;
-constexpr uint32_t kEeV = 8;         // edges per warp
 constexpr uint32_t kEePairBuf = 288;
 constexpr uint32_t kEeEdgeBits = 29;  // buffered pairs: edge of the cluster << 29 | candidate edge
+template <uint32_t kEeV>
 struct EeWarp {
   uint32_t end[kScCells], beg[kScCells];  // (see ScWarp)
   uint8_t box[kScCells];
-  float4 lo[36], hi[36];  // staged candidates: swept box, endpoints in .w
-  uint2 c[36];            // cell in the box (x, y, z bytes), index
+  float4 lo[32u + 32u / kEeV], hi[32u + 32u / kEeV];  // staged candidates: swept box, endpoints in .w
+  uint2 c[32u + 32u / kEeV];           // cell in the box (x, y, z bytes), index
   uint32_t edge[kEeV];
   union {
     uint32_t pq[kEePairBuf];
     EeSearch search;
   };
 };
+template <uint32_t kEeV>
 __global__ void __launch_bounds__(32 * kEeClusterWarps, 8) k_ee_cluster(const __grid_constant__ SCArgs s) {
-  __shared__ EeWarp sh[kEeClusterWarps];
+  __shared__ EeWarp<kEeV> sh[kEeClusterWarps];
   const uint32_t lane = threadIdx.x & 31u;
-  EeWarp& m = sh[threadIdx.x >> 5];
+  EeWarp<kEeV>& m = sh[threadIdx.x >> 5];
   const uint32_t lt_mask = (1u << lane) - 1u;
   const uint32_t at = (blockIdx.x * kEeClusterWarps + (threadIdx.x >> 5)) * kEeV;
   if (at >= s.ne) return;  // whole warp

@@ -1409,6 +1409,31 @@ struct Sim {
     });
   }
   void encode_hash(int which) { encode_hash(which, st); }
+  template <uint32_t kV>
+  void launch_sc_v(const SCArgs& a) {
+    k_sc_solve<kV><<<grid(n, kV * tcloth::kScWarps), 32 * tcloth::kScWarps, 0, st>>>(a);
+  }
+  template <uint32_t kV>
+  void launch_ee_v(const SCArgs& a, cudaStream_t ss) {
+    k_ee_cluster<kV><<<grid(ne, kV * tcloth::kEeClusterWarps), 32 * tcloth::kEeClusterWarps, 0, ss>>>(a);
+  }
+  // Elements per warp of the cluster searches.  Large clusters share more of
+  // their scan, small ones make more warps: 8 once they fill the chip several
+  // times over, fewer below.  us per pass at 1 / 2 / 4 / 8 per warp, two layers
+  // on a sphere: vertices 3,200: 21 / 23 / 32 / 45; 9,800: 53 / 51 / 46 / 70;
+  // 29,282: 149 / 120 / 109 / 111; 131,072: 1258 / 1070 / 968 / 847.  Edges
+  // (with the pairs' contact math) 9,360: 30 / 28 / 31 / 36; 28,980: 54 / 47 /
+  // 46 / 48; 87,120: 125 / 99 / 84 / 78; 391,682: 940 / 733 / 572 / 532.
+  void launch_sc_solve(const SCArgs& a) {
+    if (n < 5000u) launch_sc_v<1>(a);
+    else if (n < 40000u) launch_sc_v<4>(a);
+    else launch_sc_v<8>(a);
+  }
+  void launch_ee_cluster(const SCArgs& a, cudaStream_t ss) {
+    if (ne < 15000u) launch_ee_v<2>(a, ss);
+    else if (ne < 50000u) launch_ee_v<4>(a, ss);
+    else launch_ee_v<8>(a, ss);
+  }
   void encode_ee(const SCArgs& a, cudaStream_t ss) {
     timed("sc_solve_ee", [&] {
       TC_CK(cudaMemsetAsync(ccd_n.p, 0, (1 + tcloth::kEeSeg) * sizeof(uint32_t), ss));
@@ -1416,7 +1441,7 @@ struct Sim {
         k_ee_grouped<<<grid(ne, 32 * tcloth::kEeWarps), 32 * tcloth::kEeWarps, 0, ss>>>(a);
       } else {
         if (a.ee_cap)
-          k_ee_cluster<<<grid(ne, tcloth::kEeV * tcloth::kEeClusterWarps), 32 * tcloth::kEeClusterWarps, 0, ss>>>(a);
+          launch_ee_cluster(a, ss);
         else k_ee<<<grid(ne, 8), 256, 0, ss>>>(a);
         if (a.ee_cap) k_ee_pairs<<<tcloth::kEeSeg * tcloth::kEePairBlocks, 256, 0, ss>>>(a);
       }
@@ -1493,7 +1518,7 @@ struct Sim {
     encode_hash(0);
     timed("sc_star_box", [&] { k_star_box<<<grid(n, 256), 256, 0, st>>>(n, star_off.p, star_idx.p, x4.p, p4.p, sbox.p, st_lo.p, st_hi.p, st_mz.p); });
     if (edges_on && !fork) encode_hash(1);
-    timed("sc_solve", [&] { k_sc_solve<<<grid(n, tcloth::kScV * tcloth::kScWarps), 32 * tcloth::kScWarps, 0, st>>>(a); });
+    timed("sc_solve", [&] { launch_sc_solve(a); });
     if (a.untangle) timed("sc_untangle", [&] { k_untangle<<<grid(n, 128), 128, 0, st>>>(a); });
     if (fork) TC_CK(cudaStreamWaitEvent(st, ev_join, 0));
     if (edges_on && !fork) encode_ee(a, st);
