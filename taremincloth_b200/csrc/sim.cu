@@ -84,6 +84,34 @@ __global__ void k_extract_positions(uint32_t n, const float4* __restrict__ x4, f
 // Adaptive feedback (update_feedback_from_floats, dispatch.rs:356-429): the
 // largest per-axis displacement since the previous frame (max is order-free:
 // atomicMax on the bits of non-negative floats), then prev = x.
+// State from packed host layouts: pos, vel (or null: at rest) and w (or null:
+// the inverse masses on the device stand); thickness and layer stay.
+__global__ void k_state_in(uint32_t n, const float* __restrict__ pos, const float* __restrict__ vel,
+                           const float* __restrict__ w, float4* __restrict__ x4, float4* __restrict__ p4,
+                           float4* __restrict__ v4) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float a = pos[3 * size_t(i)], b = pos[3 * size_t(i) + 1], c = pos[3 * size_t(i) + 2];
+  x4[i] = make_float4(a, b, c, w ? w[i] : x4[i].w);
+  p4[i] = make_float4(a, b, c, p4[i].w);
+  v4[i] = vel ? make_float4(vel[3 * size_t(i)], vel[3 * size_t(i) + 1], vel[3 * size_t(i) + 2], v4[i].w)
+              : make_float4(0.f, 0.f, 0.f, v4[i].w);
+}
+// x, p and v packed as xyz, one after the other
+__global__ void k_state_out(uint32_t n, const float4* __restrict__ x4, const float4* __restrict__ p4,
+                            const float4* __restrict__ v4, float* __restrict__ out) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float4 q[3] = {x4[i], p4[i], v4[i]};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    float* o = out + 3 * (size_t(k) * n + i);
+    o[0] = q[k].x;
+    o[1] = q[k].y;
+    o[2] = q[k].z;
+  }
+}
+
 __global__ void k_fb_disp(uint32_t n, const float4* __restrict__ x4, float4* __restrict__ prev, float* out) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   float d = 0.f;
@@ -136,14 +164,14 @@ struct Mlp {
   DBuf<__nv_bfloat16> h0, h1, h2;
   DBuf<float> y;
   DBuf<__nv_bfloat16> x0, x1, x2, dz;
-  DBuf<float> z0, z1, z2, dy, dh, dx;
+  DBuf<float> z0, z1, z2, dx;
   DBuf<uint32_t> ell;  // inference: [n][16] degree, first 15 neighbours
   unsigned mp_grid = 1;
   // message-passing inference on the tcgen05 tensor cores (k_mlp_infer_mp_tc)
   // or, with tc = false, on warp-level mma.sync (k_mlp_infer_mp); err: the
   // device word a timed-out tensor-core wait sets to 2
   bool tc = true;
-  unsigned mp_grid_tc = 1, bwd_grid_tc = 1;
+  unsigned mp_grid_tc = 1, bwd_grid_tc = 1, row_grid = 1;
   int* err = nullptr;
   uint32_t adam_t = 0;
 
@@ -176,6 +204,7 @@ struct Mlp {
     TC_CK(cudaFuncSetAttribute(k_mlp_layer_bwd_tc, cudaFuncAttributePreferredSharedMemoryCarveout,
                                int(cudaSharedmemCarveoutMaxShared)));
     bwd_grid_tc = std::max(1u, std::min(unsigned(grid(n, 128)), unsigned(2 * sms)));
+    row_grid = std::max(1u, std::min(unsigned(grid(n, kWsRowWarps)), unsigned(8 * sms)));
   }
   // the ELL table of the inference kernels from the host CSR
   void set_ell(const uint32_t* h_off, const uint32_t* h_idx) {
@@ -190,7 +219,7 @@ struct Mlp {
   void alloc_train() {
     x0.alloc(size_t(n) * kWsF); x1.alloc(size_t(n) * 128); x2.alloc(size_t(n) * 128); dz.alloc(size_t(n) * kWsH);
     z0.alloc(size_t(n) * kWsH); z1.alloc(size_t(n) * kWsH); z2.alloc(size_t(n) * kWsH);
-    dy.alloc(size_t(n) * 3); dh.alloc(size_t(n) * kWsH); dx.alloc(size_t(n) * 128);
+    dx.alloc(size_t(n) * 128);
   }
   // seeded init: uniform(-1/sqrt(in), 1/sqrt(in)), the head scaled by 0.1 so
   // that an untrained network moves vertices by little; zero biases
@@ -223,8 +252,8 @@ struct Mlp {
   }
   void refresh() { k_ws_refresh<<<grid(kP_N, 256), 256, 0, st>>>(w.p, wb.p, wbt.p); }
 
-  // Y = MLP(feat); with train, keeps X1, X2, Z0..Z2 and (with target) writes
-  // dY and adds the loss to *loss.
+  // Y = MLP(feat); with train, keeps X1, X2, Z0..Z2 and (with target) adds the
+  // loss to *loss and starts the gradients: gw cleared, then the head's, and dZ2.
   void forward(const __nv_bfloat16* feat, bool train, const float* target, const float* mask, float* loss) {
     if (!n) return;
     MlpLayerArgs a{};
@@ -249,8 +278,15 @@ struct Mlp {
       a.x_out = train ? x2.p : nullptr; a.z_out = train ? z2.p : nullptr; a.h_out = h2.p;
       k_mlp_layer_fwd<<<grid(n, kWsRows), kWsFwdThreads, 0, st>>>(a);
     }
-    k_mlp_head<<<grid(n, 256), 256, 0, st>>>(n, h2.p, wb.p + kP_W3, w.p + kP_b3, y.p, target, mask, w.p + kP_YS,
-                                             1.0f / float(n), target ? dy.p : nullptr, loss);
+    if (!target) {
+      k_mlp_head<<<grid(n, 256), 256, 0, st>>>(n, h2.p, wb.p + kP_W3, w.p + kP_b3, y.p);
+      return;
+    }
+    TC_CK(cudaMemsetAsync(gw.p, 0, kP_N * sizeof(float), st));
+    // (half the blocks: each ends in 260 atomics on the same values)
+    k_mlp_head_train<<<(row_grid + 1) / 2, 32 * kWsRowWarps, 0, st>>>(
+        MlpHeadTrainArgs{n, h2.p, wb.p + kP_W3, w.p + kP_b3, z2.p, target, mask, w.p + kP_YS, 1.0f / float(n), y.p,
+                         loss, gw.p + kP_W3, gw.p + kP_b3, gw.p + kP_b2, dz.p});
   }
   // inference: layer 0 from the given features (feat) or computed from fa
   // (then p is kept in ppred first); the head is fused into the last layer,
@@ -274,28 +310,29 @@ struct Mlp {
     a.local_len = local_len;
     mp();
   }
-  // gradients of the loss of the last forward(train, target) into gw (layer
+  // the other gradients of the loss of the last forward(train, target) into gw (layer
   // 0's input is the scaled copy x0 that forward kept)
   void backward() {
-    TC_CK(cudaMemsetAsync(gw.p, 0, kP_N * sizeof(float), st));
-    if (!n) return;
-    const unsigned gh = grid(size_t(n) * kWsH, 256), gt = grid(n, kWsRows);
-    k_mlp_head_bwd<<<grid(n, 256), 256, 0, st>>>(n, h2.p, wb.p + kP_W3, dy.p, dh.p, gw.p + kP_W3, gw.p + kP_b3);
-    k_mlp_act_bwd<<<gh, 256, 0, st>>>(n, dh.p, z2.p, dz.p, gw.p + kP_b2);
+    if (!n) {
+      TC_CK(cudaMemsetAsync(gw.p, 0, kP_N * sizeof(float), st));
+      return;
+    }
+    const unsigned gt = grid(n, kWsRows);
     auto bwd128 = [&](const __nv_bfloat16* x, uint32_t wo) {
       if (tc)
         k_mlp_layer_bwd_tc<<<bwd_grid_tc, 256, kWsBwdSmem, st>>>(
-            MlpBwdTcArgs{n, x, dz.p, wb.p + wo, gw.p + wo, dx.p, err});
+            MlpBwdTcArgs{n, x, dz.p, wb.p + wo, gw.p + wo, dx.p, adj_off, err});
       else
-        k_mlp_layer_bwd<<<gt, 128, 0, st>>>(MlpBwdArgs{n, 128, x, dz.p, wb.p + wo, gw.p + wo, dx.p});
+        k_mlp_layer_bwd<<<gt, 128, 0, st>>>(MlpBwdArgs{n, 128, x, dz.p, wb.p + wo, gw.p + wo, dx.p, adj_off});
+    };
+    auto below = [&](const float* z, uint32_t bo) {
+      k_mlp_agg_act_bwd<<<row_grid, 32 * kWsRowWarps, 0, st>>>(n, dx.p, adj_off, adj_idx, z, dz.p, gw.p + bo);
     };
     bwd128(x2.p, kP_W2);
-    k_mlp_agg_bwd<<<gh, 256, 0, st>>>(n, dx.p, adj_off, adj_idx, dh.p);
-    k_mlp_act_bwd<<<gh, 256, 0, st>>>(n, dh.p, z1.p, dz.p, gw.p + kP_b1);
+    below(z1.p, kP_b1);
     bwd128(x1.p, kP_W1);
-    k_mlp_agg_bwd<<<gh, 256, 0, st>>>(n, dx.p, adj_off, adj_idx, dh.p);
-    k_mlp_act_bwd<<<gh, 256, 0, st>>>(n, dh.p, z0.p, dz.p, gw.p + kP_b0);
-    k_mlp_layer_bwd<<<gt, 128, 0, st>>>(MlpBwdArgs{n, kWsF, x0.p, dz.p, wb.p + kP_W0, gw.p + kP_W0, nullptr});
+    below(z0.p, kP_b0);
+    k_mlp_layer0_dw<<<std::min(gt, (row_grid + 3) / 4), 128, 0, st>>>(n, x0.p, dz.p, gw.p + kP_W0);
   }
   // Normalizer from `rows` recorded rows (features, targets, free mask): FS =
   // 1 / RMS of each feature, YS = RMS of the target components, over the
@@ -997,6 +1034,60 @@ struct Sim {
     v4.upload(hv, st);
     if (ws.ready) TC_CK(cudaMemsetAsync(ws.dprev.p, 0, size_t(n) * sizeof(float4), st));
     TC_CK(cudaStreamSynchronize(st));
+    w_current = false;
+  }
+
+  // The state from host arrays (tc_set_positions_and_velocities) and back
+  // (tc_get_state): the packed arrays cross the bus and are spread out on the
+  // device, through the star boxes' buffer, which only a self-collision pass
+  // uses and every pass fills anew.  Inverse masses go along when they may have
+  // changed.  (Building and reading padded arrays on the host took 3.8 ms of a
+  // 131,072-vertex frame.)
+  bool w_current = false;
+  static constexpr uint32_t kSmallState = 16384;
+  std::vector<float> state_h;
+  void seek(const float* pos, const float* vel) {
+    float* buf = reinterpret_cast<float*>(sbox.p);
+    const size_t n3 = size_t(n) * 3;
+    if (n <= kSmallState && vel) {  // one copy: its latency is the cost
+      state_h.resize(3 * n3);
+      std::memcpy(state_h.data(), pos, n3 * sizeof(float));
+      std::memcpy(state_h.data() + n3, vel, n3 * sizeof(float));
+      TC_CK(cudaMemcpyAsync(buf, state_h.data(), 2 * n3 * sizeof(float), cudaMemcpyHostToDevice, st));
+    } else {
+      TC_CK(cudaMemcpyAsync(buf, pos, n3 * sizeof(float), cudaMemcpyHostToDevice, st));
+      if (vel) TC_CK(cudaMemcpyAsync(buf + n3, vel, n3 * sizeof(float), cudaMemcpyHostToDevice, st));
+    }
+    if (!w_current) {
+      std::vector<float> w(orig_w);
+      for (const auto& kv : pins) w[kv.first] = orig_w[kv.first] * (1.f - clamp_w(kv.second.weight));
+      TC_CK(cudaMemcpyAsync(buf + 2 * n3, w.data(), size_t(n) * sizeof(float), cudaMemcpyHostToDevice, st));
+    }
+    k_state_in<<<grid(n, 256), 256, 0, st>>>(n, buf, vel ? buf + n3 : nullptr, w_current ? nullptr : buf + 2 * n3,
+                                              x4.p, p4.p, v4.p);
+    TC_CK(cudaGetLastError());
+    if (ws.ready) TC_CK(cudaMemsetAsync(ws.dprev.p, 0, size_t(n) * sizeof(float4), st));
+    TC_CK(cudaStreamSynchronize(st));
+    w_current = true;
+  }
+  void get_state(float* x, float* p, float* v) {
+    if (n == 0) return;
+    float* buf = reinterpret_cast<float*>(sbox.p);
+    k_state_out<<<grid(n, 256), 256, 0, st>>>(n, x4.p, p4.p, v4.p, buf);
+    TC_CK(cudaGetLastError());
+    const size_t n3 = size_t(n) * 3;
+    float* out[3] = {x, p, v};
+    if (n <= kSmallState) {
+      state_h.resize(3 * n3);
+      TC_CK(cudaMemcpyAsync(state_h.data(), buf, 3 * n3 * sizeof(float), cudaMemcpyDeviceToHost, st));
+      TC_CK(cudaStreamSynchronize(st));
+      for (int k = 0; k < 3; ++k)
+        if (out[k]) std::memcpy(out[k], state_h.data() + k * n3, n3 * sizeof(float));
+      return;
+    }
+    for (int k = 0; k < 3; ++k)
+      if (out[k]) TC_CK(cudaMemcpyAsync(out[k], buf + k * n3, n3 * sizeof(float), cudaMemcpyDeviceToHost, st));
+    TC_CK(cudaStreamSynchronize(st));
   }
 
   void upload_dist() {
@@ -1294,6 +1385,7 @@ struct Sim {
     cl_stale = true;
     st_stale = true;
     rs_pins_stale = true;
+    w_current = false;
     std::vector<uint32_t> v;
     std::vector<float4> t;
     for (const auto& kv : pins) {
@@ -1309,6 +1401,7 @@ struct Sim {
     TC_CK(cudaMemcpyAsync(reinterpret_cast<char*>(x4.p) + size_t(v) * sizeof(float4) + 12, &w, 4,
                           cudaMemcpyHostToDevice, st));
     TC_CK(cudaStreamSynchronize(st));
+    w_current = false;
   }
   static float clamp_w(float w) { return std::isfinite(w) ? std::fmin(std::fmax(w, 0.f), 1.f) : 0.f; }
 
@@ -3063,12 +3156,7 @@ tc_status tc_set_positions_and_velocities(tc_sim* s, const float* pos, const flo
   return guard([&] {
     Sim& m = S(s);
     if (m.n == 0 || n != m.n || !pos) return;  // the reference ignores a length mismatch
-    std::vector<float> w(m.n);
-    for (uint32_t i = 0; i < m.n; ++i) {
-      auto it = m.pins.find(i);
-      w[i] = it != m.pins.end() ? m.orig_w[i] * (1.f - Sim::clamp_w(it->second.weight)) : m.orig_w[i];
-    }
-    m.upload_vertices(pos, vel, w.data());
+    m.seek(pos, vel);
   });
 }
 
@@ -3555,16 +3643,7 @@ tc_status tc_get_cell_size(tc_sim* s, float* cell) {
 tc_status tc_get_state(tc_sim* s, float* x, float* p, float* v) {
   return guard([&] {
     Sim& m = S(s);
-    std::vector<float4> hx(m.n), hp(m.n), hv(m.n);
-    TC_CK(cudaMemcpyAsync(hx.data(), m.x4.p, m.n * sizeof(float4), cudaMemcpyDeviceToHost, m.st));
-    TC_CK(cudaMemcpyAsync(hp.data(), m.p4.p, m.n * sizeof(float4), cudaMemcpyDeviceToHost, m.st));
-    TC_CK(cudaMemcpyAsync(hv.data(), m.v4.p, m.n * sizeof(float4), cudaMemcpyDeviceToHost, m.st));
-    TC_CK(cudaStreamSynchronize(m.st));
-    for (uint32_t i = 0; i < m.n; ++i) {
-      if (x) { x[3 * i] = hx[i].x; x[3 * i + 1] = hx[i].y; x[3 * i + 2] = hx[i].z; }
-      if (p) { p[3 * i] = hp[i].x; p[3 * i + 1] = hp[i].y; p[3 * i + 2] = hp[i].z; }
-      if (v) { v[3 * i] = hv[i].x; v[3 * i + 1] = hv[i].y; v[3 * i + 2] = hv[i].z; }
-    }
+    m.get_state(x, p, v);
   });
 }
 tc_status tc_get_distance_constraints(tc_sim* s, uint32_t* v01, float* par, uint32_t* off, uint32_t* cnt) {

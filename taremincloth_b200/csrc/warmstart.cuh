@@ -254,79 +254,165 @@ __global__ void __launch_bounds__(kWsFwdThreads) k_mlp_layer_fwd(MlpLayerArgs a)
   }
 }
 
-// Head: Y = H2 W3 + b3 (fp32 accumulation of bf16 products).  With targets,
-// also dY = 2 (Y - T / YS) m / (3 n) (mean squared error against the
-// normalised target, mask m of free vertices) and the loss.
+// Head: Y = H2 W3 + b3 (fp32 accumulation of bf16 products), without targets.
 __global__ void k_mlp_head(uint32_t n, const __nv_bfloat16* __restrict__ h2, const __nv_bfloat16* __restrict__ w3,
-                           const float* __restrict__ b3, float* __restrict__ y, const float* __restrict__ target,
-                           const float* __restrict__ mask, const float* __restrict__ yscale, float inv_count,
-                           float* __restrict__ dy, float* __restrict__ loss) {
+                           const float* __restrict__ b3, float* __restrict__ y) {
   const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  float l = 0.f;
-  const float ys = out_scale(yscale);
-  if (v < n) {
+  if (v >= n) return;
+  for (int c = 0; c < 3; ++c) {
+    float s = 0.f;
+    for (int k = 0; k < kWsH; ++k) s += __bfloat162float(h2[size_t(v) * kWsH + k]) * __bfloat162float(w3[k * 3 + c]);
+    y[size_t(v) * 3 + c] = s + b3[c];
+  }
+}
+
+// The per-row passes of training.  A warp takes a row at a time, lane l the
+// columns 2l and 2l + 1, so that every access is one coalesced line; what is
+// summed over the rows (bias and head gradients, loss) stays in the lane's
+// registers and goes through shared memory to one atomic per block and value.
+// (One thread per row or element, with shared-memory atomics per value, took
+// 488 us for the head and 69 us per activation on 75,000 rows.)
+constexpr int kWsRowWarps = 8;
+// sums of the block's warps' values (out[0 .. kWsH) += the two columns of each lane)
+__device__ __forceinline__ void add_columns(float a0, float a1, float* sh, float* out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  sh[warp * kWsH + 2 * lane] = a0;
+  sh[warp * kWsH + 2 * lane + 1] = a1;
+  __syncthreads();
+  if (threadIdx.x < kWsH) {
+    float t = 0.f;
+    for (int w = 0; w < kWsRowWarps; ++w) t += sh[w * kWsH + threadIdx.x];
+    atomicAdd(out + threadIdx.x, t);
+  }
+  __syncthreads();
+}
+__device__ __forceinline__ float warp_sum(float v) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ float2 bf16x2(uint32_t u) {
+  return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xFFFF0000u));
+}
+__device__ __forceinline__ void store_dz(__nv_bfloat16* dz, size_t row, int lane, float g0, float g1) {
+  reinterpret_cast<uint32_t*>(dz + row * kWsH)[lane] = pack_bf16(__float2bfloat16(g0), __float2bfloat16(g1));
+}
+
+// Head of a training step: Y = H2 W3 + b3, the loss (mean squared error of Y
+// against the normalised target T / YS, mask m of free vertices) with its
+// gradient dY = 2 (Y - T / YS) m / (3 n), dW3 += H2^T dY, db3 += sum dY, and
+// dZ2 = (dY W3^T) SiLU'(Z2), rounded to bf16 for the tensor-core GEMMs, with
+// db2 += sum dZ2.
+struct MlpHeadTrainArgs {
+  uint32_t n;
+  const __nv_bfloat16* h2;
+  const __nv_bfloat16* w3;
+  const float *b3, *z2, *target, *mask, *yscale;
+  float inv_count;
+  float *y, *loss, *dw3, *db3, *db2;
+  __nv_bfloat16* dz;
+};
+__global__ void __launch_bounds__(32 * kWsRowWarps) k_mlp_head_train(MlpHeadTrainArgs a) {
+  __shared__ float sh[kWsRowWarps * kWsH];
+  const int lane = threadIdx.x & 31;
+  const uint32_t warps = gridDim.x * kWsRowWarps;
+  float w[2][3], dw[2][3] = {}, db[2] = {}, db3[3] = {}, loss = 0.f;
+  for (int q = 0; q < 2; ++q)
+    for (int c = 0; c < 3; ++c) w[q][c] = __bfloat162float(a.w3[(2 * lane + q) * 3 + c]);
+  const float ys = out_scale(a.yscale);
+  const float b3[3] = {a.b3[0], a.b3[1], a.b3[2]};
+#pragma unroll 2
+  for (uint32_t v = blockIdx.x * kWsRowWarps + (threadIdx.x >> 5); v < a.n; v += warps) {
+    const float2 h = bf16x2(__ldg(reinterpret_cast<const uint32_t*>(a.h2 + size_t(v) * kWsH) + lane));
+    const float2 z = __ldg(reinterpret_cast<const float2*>(a.z2 + size_t(v) * kWsH) + lane);
+    const float m = a.mask ? __ldg(a.mask + v) : 1.0f;
+    float d[3];
+    float s = 0.f;
+#pragma unroll
     for (int c = 0; c < 3; ++c) {
-      float s = 0.f;
-      for (int k = 0; k < kWsH; ++k) s += __bfloat162float(h2[size_t(v) * kWsH + k]) * __bfloat162float(w3[k * 3 + c]);
-      s += b3[c];
-      y[size_t(v) * 3 + c] = s;
-      if (target) {
-        const float m = mask ? mask[v] : 1.0f;
-        const float d = (s - target[size_t(v) * 3 + c] / ys) * m;
-        dy[size_t(v) * 3 + c] = 2.0f * d * inv_count / 3.0f;
-        l += d * d;
+      const float t = warp_sum(h.x * w[0][c] + h.y * w[1][c]) + b3[c];
+      if (lane == c) s = t;
+    }
+    // lane c < 3 holds component c
+    float e = 0.f;
+    if (lane < 3) {
+      a.y[size_t(v) * 3 + lane] = s;
+      e = (s - __ldg(a.target + size_t(v) * 3 + lane) / ys) * m;
+      loss += e * e;
+    }
+    const float dl = 2.0f * e * a.inv_count / 3.0f;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      d[c] = __shfl_sync(0xffffffffu, dl, c);
+      dw[0][c] += h.x * d[c];
+      dw[1][c] += h.y * d[c];
+      db3[c] += d[c];
+    }
+    const float g0 = (d[0] * w[0][0] + d[1] * w[0][1] + d[2] * w[0][2]) * silu_grad(z.x);
+    const float g1 = (d[0] * w[1][0] + d[1] * w[1][1] + d[2] * w[1][2]) * silu_grad(z.y);
+    store_dz(a.dz, v, lane, g0, g1);
+    db[0] += g0;
+    db[1] += g1;
+  }
+  add_columns(db[0], db[1], sh, a.db2);
+  for (int c = 0; c < 3; ++c) {  // dW3 is [64][3]
+    const int warp = threadIdx.x >> 5;
+    sh[warp * kWsH + 2 * lane] = dw[0][c];
+    sh[warp * kWsH + 2 * lane + 1] = dw[1][c];
+    __syncthreads();
+    if (threadIdx.x < kWsH) {
+      float t = 0.f;
+      for (int q = 0; q < kWsRowWarps; ++q) t += sh[q * kWsH + threadIdx.x];
+      atomicAdd(a.dw3 + threadIdx.x * 3 + c, t);
+    }
+    __syncthreads();
+  }
+  // (every lane of a warp holds the same db3; lanes 0 to 2 their component's loss)
+  loss = warp_sum(loss);
+  if (lane < 4) sh[(threadIdx.x >> 5) * 4 + lane] = lane < 3 ? db3[lane == 0 ? 0 : lane == 1 ? 1 : 2] : loss;
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    float t = 0.f;
+    for (int q = 0; q < kWsRowWarps; ++q) t += sh[q * 4 + threadIdx.x];
+    if (threadIdx.x < 3) atomicAdd(a.db3 + threadIdx.x, t);
+    else atomicAdd(a.loss, t * a.inv_count / 3.0f);
+  }
+}
+
+// Backward through the neighbour mean and the activation of the layer below:
+// dH[j] = dX[j][0:64] + sum_{i in N(j)} dX[i][64:128] / deg(i) (the adjacency
+// is symmetric, so the transpose of the mean is a gather; the layer's backward
+// has divided by deg(i)), dZ = dH SiLU'(Z) rounded to bf16, db += sum dZ.
+__global__ void __launch_bounds__(32 * kWsRowWarps) k_mlp_agg_act_bwd(uint32_t n, const float* __restrict__ dx,
+                                                                      const uint32_t* __restrict__ adj_off,
+                                                                      const uint32_t* __restrict__ adj_idx,
+                                                                      const float* __restrict__ z,
+                                                                      __nv_bfloat16* __restrict__ dz,
+                                                                      float* __restrict__ db) {
+  __shared__ float sh[kWsRowWarps * kWsH];
+  const int lane = threadIdx.x & 31;
+  const uint32_t warps = gridDim.x * kWsRowWarps;
+  float d0 = 0.f, d1 = 0.f;
+  for (uint32_t j = blockIdx.x * kWsRowWarps + (threadIdx.x >> 5); j < n; j += warps) {
+    const uint32_t b = __ldg(adj_off + j), e = __ldg(adj_off + j + 1);
+    const float2 zz = __ldg(reinterpret_cast<const float2*>(z + size_t(j) * kWsH) + lane);
+    float2 s = __ldg(reinterpret_cast<const float2*>(dx + size_t(j) * 128) + lane);
+    for (uint32_t q0 = b; q0 < e; q0 += 32u) {
+      const uint32_t cnt = min(e - q0, 32u);
+      const uint32_t mine = uint32_t(lane) < cnt ? __ldg(adj_idx + q0 + lane) : 0u;
+#pragma unroll 4
+      for (uint32_t q = 0; q < cnt; ++q) {
+        const uint32_t i = __shfl_sync(0xffffffffu, mine, int(q));
+        const float2 t = __ldg(reinterpret_cast<const float2*>(dx + size_t(i) * 128 + kWsH) + lane);
+        s.x += t.x;
+        s.y += t.y;
       }
     }
+    const float g0 = s.x * silu_grad(zz.x), g1 = s.y * silu_grad(zz.y);
+    store_dz(dz, j, lane, g0, g1);
+    d0 += g0;
+    d1 += g1;
   }
-  if (target) {
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, l * inv_count / 3.0f);
-  }
-}
-
-// Head backward: dH2 = dY W3^T (fp32), dW3 += H2^T dY, db3 += sum dY.
-__global__ void k_mlp_head_bwd(uint32_t n, const __nv_bfloat16* __restrict__ h2, const __nv_bfloat16* __restrict__ w3,
-                               const float* __restrict__ dy, float* __restrict__ dh2, float* __restrict__ dw3,
-                               float* __restrict__ db3) {
-  __shared__ float s_dw[kWsH * 3];
-  __shared__ float s_db[3];
-  for (int e = threadIdx.x; e < kWsH * 3; e += blockDim.x) s_dw[e] = 0.f;
-  if (threadIdx.x < 3) s_db[threadIdx.x] = 0.f;
-  __syncthreads();
-  const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v < n) {
-    const float d0 = dy[size_t(v) * 3], d1 = dy[size_t(v) * 3 + 1], d2 = dy[size_t(v) * 3 + 2];
-    for (int k = 0; k < kWsH; ++k) {
-      const float w0 = __bfloat162float(w3[k * 3]), w1 = __bfloat162float(w3[k * 3 + 1]), w2 = __bfloat162float(w3[k * 3 + 2]);
-      dh2[size_t(v) * kWsH + k] = d0 * w0 + d1 * w1 + d2 * w2;
-      const float h = __bfloat162float(h2[size_t(v) * kWsH + k]);
-      atomicAdd(&s_dw[k * 3], h * d0);
-      atomicAdd(&s_dw[k * 3 + 1], h * d1);
-      atomicAdd(&s_dw[k * 3 + 2], h * d2);
-    }
-    atomicAdd(&s_db[0], d0);
-    atomicAdd(&s_db[1], d1);
-    atomicAdd(&s_db[2], d2);
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < kWsH * 3; e += blockDim.x) atomicAdd(&dw3[e], s_dw[e]);
-  if (threadIdx.x < 3) atomicAdd(&db3[threadIdx.x], s_db[threadIdx.x]);
-}
-
-// dZ = dH * SiLU'(Z), rounded to bf16 for the tensor-core GEMMs; db += sum dZ.
-__global__ void k_mlp_act_bwd(uint32_t n, const float* __restrict__ dh, const float* __restrict__ z,
-                              __nv_bfloat16* __restrict__ dz, float* __restrict__ db) {
-  __shared__ float s_db[kWsH];
-  if (threadIdx.x < kWsH) s_db[threadIdx.x] = 0.f;
-  __syncthreads();
-  const size_t e = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e < size_t(n) * kWsH) {
-    const float g = dh[e] * silu_grad(z[e]);
-    dz[e] = __float2bfloat16(g);
-    atomicAdd(&s_db[e % kWsH], g);
-  }
-  __syncthreads();
-  if (threadIdx.x < kWsH) atomicAdd(&db[threadIdx.x], s_db[threadIdx.x]);
+  add_columns(d0, d1, sh, db);
 }
 
 // Weight gradient dW[kin][64] += X^T dZ over a 64-row tile (tensor cores),
@@ -338,7 +424,8 @@ struct MlpBwdArgs {
   const __nv_bfloat16* dz;   // [n][64]
   const __nv_bfloat16* w;    // [kin][64] (row-major weights = n-major for dZ W^T)
   float* dw;                 // [kin][64]
-  float* dx;                 // [n][kin] or null
+  float* dx;                 // [n][kin] or null; columns 64.. divided by the row's degree
+  const uint32_t* adj_off;
 };
 __global__ void __launch_bounds__(128) k_mlp_layer_bwd(MlpBwdArgs a) {
   __shared__ __align__(16) __nv_bfloat16 xs[kWsRows][128 + 8];
@@ -390,9 +477,65 @@ __global__ void __launch_bounds__(128) k_mlp_layer_bwd(MlpBwdArgs a) {
     }
     for (int q = 0; q < 4; ++q) {
       const int r = warp * 16 + g + (q >> 1) * 8, c = nt * 8 + 2 * t + (q & 1);
-      if (row0 + r < a.n) a.dx[size_t(row0 + r) * kin + c] = acc[q];
+      if (row0 + r < a.n)
+        a.dx[size_t(row0 + r) * kin + c] =
+            c < kWsH ? acc[q] : acc[q] / float(a.adj_off[row0 + r + 1] - a.adj_off[row0 + r]);
     }
   }
+}
+
+// Weight gradient of layer 0, dW[16][64] += X^T dZ (below the tcgen05 MMA's M =
+// 64, so on mma.sync).  Persistent blocks: every warp keeps its sum over its
+// rows, 16 at a time, in registers, and a block adds to the global sum once (a
+// block per 64 rows, each with 1,024 atomics on the same values, took 34 us on
+// 68,000 rows).
+__global__ void __launch_bounds__(128) k_mlp_layer0_dw(uint32_t n, const __nv_bfloat16* __restrict__ x,
+                                                       const __nv_bfloat16* __restrict__ dz, float* __restrict__ dw) {
+  __shared__ __align__(16) __nv_bfloat16 xs[4][16][kWsF + 8];
+  __shared__ __align__(16) __nv_bfloat16 ds[4][16][kWsH + 8];
+  __shared__ float sum[kWsF * kWsH];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int e = threadIdx.x; e < kWsF * kWsH; e += blockDim.x) sum[e] = 0.f;
+  float acc[8][4] = {};
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  for (uint32_t r0 = (blockIdx.x * 4u + warp) * 16u; r0 < n; r0 += gridDim.x * 64u) {
+    __syncwarp();
+    {  // 16 rows x 2 and x 8 chunks of 16 bytes
+      const uint32_t r = lane >> 1, c = lane & 1;
+      *reinterpret_cast<uint4*>(&xs[warp][r][c * 8]) =
+          r0 + r < n ? __ldg(reinterpret_cast<const uint4*>(x + size_t(r0 + r) * kWsF) + c) : zero;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t e = q * 32 + lane, r = e >> 3, c = e & 7;
+      *reinterpret_cast<uint4*>(&ds[warp][r][c * 8]) =
+          r0 + r < n ? __ldg(reinterpret_cast<const uint4*>(dz + size_t(r0 + r) * kWsH) + c) : zero;
+    }
+    __syncwarp();
+    uint32_t af[4];
+    load_at_frag(af, &xs[warp][0][0], kWsF + 8, 0, 0, lane);
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+      uint32_t bf[2];
+      load_bk_frag(bf, &ds[warp][0][0], kWsH + 8, nt * 8, 0, lane);
+      mma_bf16_16816(acc[nt], af, bf);
+    }
+  }
+  __syncthreads();
+  const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      atomicAdd(&sum[(g + (q >> 1) * 8) * kWsH + nt * 8 + 2 * t + (q & 1)], acc[nt][q]);
+  __syncthreads();
+  for (int e = threadIdx.x; e < kWsF * kWsH; e += blockDim.x) atomicAdd(dw + e, sum[e]);
+}
+
+// p[0..3] += v[0..3], p 16-byte aligned
+__device__ __forceinline__ void red_add4(float* p, const float* v) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3])
+               : "memory");
 }
 
 // Backward of a 128-wide layer on the tcgen05 tensor cores.  Persistent CTAs
@@ -412,7 +555,8 @@ struct MlpBwdTcArgs {
   const __nv_bfloat16* dz;  // [n][64]
   const __nv_bfloat16* w;   // [128][64] row-major weights
   float* dw;                // [128][64], added to
-  float* dx;                // [n][128] or null
+  float* dx;                // [n][128] or null; columns 64.. divided by the row's degree
+  const uint32_t* adj_off;
   int* err;
 };
 constexpr uint32_t kWsBwdCols = 256;
@@ -492,11 +636,19 @@ __global__ void __launch_bounds__(256, 2) k_mlp_layer_bwd_tc(MlpBwdTcArgs a) {
 #pragma unroll
       for (int c0 = 0; c0 < 64; c0 += 32) {
         float z[32];
-        const uint32_t taddr = tbase + (uint32_t(quad * 32) << 16) + 64u + uint32_t(half * 64 + c0);
+        // 32 columns of the row itself, then 32 of its neighbours' mean, so
+        // that both halves of the warps share the divisions
+        const int col = 2 * c0 + half * 32;
+        const uint32_t taddr = tbase + (uint32_t(quad * 32) << 16) + 64u + uint32_t(col);
         tmem_ld16(taddr, z);
         tmem_ld16(taddr + 16, z + 16);
         if (v < a.n) {
-          float4* o = reinterpret_cast<float4*>(a.dx + size_t(v) * 128 + half * 64 + c0);
+          float4* o = reinterpret_cast<float4*>(a.dx + size_t(v) * 128 + col);
+          if (c0) {
+            const float deg = float(__ldg(a.adj_off + v + 1) - __ldg(a.adj_off + v));
+#pragma unroll
+            for (int q = 0; q < 32; ++q) z[q] /= deg;
+          }
 #pragma unroll
           for (int q = 0; q < 8; ++q) o[q] = make_float4(z[4 * q], z[4 * q + 1], z[4 * q + 2], z[4 * q + 3]);
         }
@@ -510,8 +662,9 @@ __global__ void __launch_bounds__(256, 2) k_mlp_layer_bwd_tc(MlpBwdTcArgs a) {
     const uint32_t taddr = tbase + (uint32_t(quad * 32) << 16) + uint32_t(half * 32);
     tmem_ld16(taddr, z);
     tmem_ld16(taddr + 16, z + 16);
+    // (four sums an instruction: 296 CTAs add to the same 8,192 values)
 #pragma unroll
-    for (int k = 0; k < 32; ++k) atomicAdd(&a.dw[c * kWsH + half * 32 + k], z[k]);
+    for (int k = 0; k < 32; k += 4) red_add4(a.dw + c * kWsH + half * 32 + k, z + k);
   }
   if (!ok) {
     if (tid == 0 && a.err) atomicExch(a.err, 2);
@@ -520,22 +673,6 @@ __global__ void __launch_bounds__(256, 2) k_mlp_layer_bwd_tc(MlpBwdTcArgs a) {
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tbase, kWsBwdCols);
-}
-
-// dH_prev[j] = dX[j][0:64] + sum_{i in N(j)} dX[i][64:128] / deg(i)
-// (the adjacency is symmetric, so the transpose of the mean is a gather).
-__global__ void k_mlp_agg_bwd(uint32_t n, const float* __restrict__ dx, const uint32_t* __restrict__ adj_off,
-                              const uint32_t* __restrict__ adj_idx, float* __restrict__ dh_prev) {
-  const size_t e = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e >= size_t(n) * kWsH) return;
-  const uint32_t j = uint32_t(e / kWsH), c = uint32_t(e % kWsH);
-  float s = dx[size_t(j) * 128 + c];
-  for (uint32_t q = adj_off[j]; q < adj_off[j + 1]; ++q) {
-    const uint32_t i = adj_idx[q];
-    const uint32_t deg = adj_off[i + 1] - adj_off[i];
-    s += dx[size_t(i) * 128 + kWsH + c] / float(deg);
-  }
-  dh_prev[e] = s;
 }
 
 // Adam on fp32 master weights; refreshes the bf16 copy (optionally transposed
