@@ -1558,6 +1558,9 @@ struct Sim {
   // phase only at the first substep of the frame, the narrow phase over the
   // cached slots at every substep.  With the final fallback on (default) the
   // last substep runs the direct pass on a fresh hash instead.
+  // (a warp per block: the scans' lengths differ, and the 2,500 warps of 80,000
+  // vertices are 1.4 waves; 128 threads: 12.4 ms a frame, 64: 12.1, 32: 11.8)
+  static constexpr unsigned kPairBlock = 32;
   void encode_pair_self_collision(bool run_ee, bool rebuild, float dt) {
     SCArgs a = sc_args();
     const PairArgs p = pair_args(dt);
@@ -1568,14 +1571,14 @@ struct Sim {
       timed("pair_collect", [&] {
         k_pair_horizon<<<grid(n, 256), 256, 0, st>>>(n, v4.p, p);
         if (profiling) {
-          k_pair_collect<0><<<grid(n, 128), 128, 0, st>>>(a, p);
-          k_pair_collect<1><<<grid(n, 128), 128, 0, st>>>(a, p);
+          k_pair_collect<0><<<grid(n, kPairBlock), kPairBlock, 0, st>>>(a, p);
+          k_pair_collect<1><<<grid(n, kPairBlock), kPairBlock, 0, st>>>(a, p);
         } else {  // the two lists are independent: the edge-edge scan runs beside
           TC_CK(cudaEventRecord(ev_fork, st));
           TC_CK(cudaStreamWaitEvent(st2, ev_fork, 0));
-          k_pair_collect<1><<<grid(n, 128), 128, 0, st2>>>(a, p);
+          k_pair_collect<1><<<grid(n, kPairBlock), kPairBlock, 0, st2>>>(a, p);
           TC_CK(cudaEventRecord(ev_join, st2));
-          k_pair_collect<0><<<grid(n, 128), 128, 0, st>>>(a, p);
+          k_pair_collect<0><<<grid(n, kPairBlock), kPairBlock, 0, st>>>(a, p);
           TC_CK(cudaStreamWaitEvent(st, ev_join, 0));
         }
       });
@@ -4274,18 +4277,38 @@ bool valid_tri(const int32_t* t, size_t nv) {
 void close_open_loops(std::vector<float>& verts, std::vector<int32_t>& tris, std::vector<std::vector<float>>& weights) {
   const size_t nv = verts.size() / 3, nt = tris.size() / 3;
   if (nt < 4 || nv < 4) return;
-  std::map<std::pair<int32_t, int32_t>, uint32_t> ecount;
-  std::vector<std::array<int32_t, 3>> existing;
+  // uses of each undirected edge, in an open-addressing table
+  size_t slots = 16;
+  while (slots < nt * 6) slots *= 2;
+  std::vector<uint64_t> ekey(slots, ~0ull);
+  std::vector<uint32_t> ecount(slots, 0u);
+  auto edge_slot = [&](int32_t a, int32_t b) {
+    const uint64_t k = uint64_t(uint32_t(std::min(a, b))) << 32 | uint32_t(std::max(a, b));
+    size_t h = size_t((k * 0x9E3779B97F4A7C15ull) >> 20) & (slots - 1);
+    while (ekey[h] != ~0ull && ekey[h] != k) h = (h + 1) & (slots - 1);
+    ekey[h] = k;
+    return h;
+  };
   for (size_t t = 0; t < nt; ++t) {
     const int32_t* q = &tris[3 * t];
     if (!valid_tri(q, nv)) continue;
-    std::array<int32_t, 3> k{q[0], q[1], q[2]};
-    std::sort(k.begin(), k.end());
-    existing.push_back(k);
-    const int32_t e[3][2] = {{q[0], q[1]}, {q[1], q[2]}, {q[2], q[0]}};
-    for (auto& x : e) ecount[{std::min(x[0], x[1]), std::max(x[0], x[1])}] += 1;
+    for (int e = 0; e < 3; ++e) ++ecount[edge_slot(q[e], q[(e + 1) % 3])];
   }
-  std::sort(existing.begin(), existing.end());
+  // the triangles as sorted triples, for the loops of three vertices
+  std::vector<std::array<int32_t, 3>> existing;
+  bool have_existing = false;
+  auto list_existing = [&] {
+    if (have_existing) return;
+    have_existing = true;
+    for (size_t t = 0; t < nt; ++t) {
+      const int32_t* q = &tris[3 * t];
+      if (!valid_tri(q, nv)) continue;
+      std::array<int32_t, 3> k{q[0], q[1], q[2]};
+      std::sort(k.begin(), k.end());
+      existing.push_back(k);
+    }
+    std::sort(existing.begin(), existing.end());
+  };
   std::vector<std::pair<int32_t, int32_t>> bedges;
   std::vector<std::array<float, 3>> bnormal;
   std::map<int32_t, std::vector<size_t>> next;
@@ -4302,7 +4325,7 @@ void close_open_loops(std::vector<float>& verts, std::vector<int32_t>& tris, std
     h_normalize(cr, tn);
     const int32_t e[3][2] = {{q[0], q[1]}, {q[1], q[2]}, {q[2], q[0]}};
     for (auto& x : e) {
-      if (ecount[{std::min(x[0], x[1]), std::max(x[0], x[1])}] == 1) {
+      if (ecount[edge_slot(x[0], x[1])] == 1) {
         next[x[0]].push_back(bedges.size());
         bedges.push_back({x[0], x[1]});
         bnormal.push_back({tn[0], tn[1], tn[2]});
@@ -4358,6 +4381,7 @@ void close_open_loops(std::vector<float>& verts, std::vector<int32_t>& tris, std
     for (size_t ei : le) ds += (bnormal[ei][0] * capn[0] + bnormal[ei][1] * capn[1]) + bnormal[ei][2] * capn[2];
     if (ds / float(std::max<size_t>(le.size(), 1)) <= -0.85f) continue;
     if (k == 3) {
+      list_existing();
       std::array<int32_t, 3> key{lv[0], lv[1], lv[2]};
       std::sort(key.begin(), key.end());
       if (std::binary_search(existing.begin(), existing.end(), key)) continue;
@@ -4581,6 +4605,10 @@ MeshBakeSetup mesh_bake_setup(const std::vector<float>& verts, const std::vector
                                      make_float4(0, 1, 0, 0)});
   return S;
 }
+tcloth::MeshBakeParams mesh_bake_params(const MeshBakeSetup& S, uint32_t ntri) {
+  return tcloth::MeshBakeParams{{S.lo[0], S.lo[1], S.lo[2]}, {S.hi[0], S.hi[1], S.hi[2]}, S.dim[0], S.dim[1], S.dim[2],
+                                ntri};
+}
 // triangles on the device with their culling spheres (one tile run)
 void mesh_bake_upload(const MeshBakeSetup& S, tcloth::BakeGpu& G, cudaStream_t st) {
   G.nt = uint32_t(S.tris.size());
@@ -4590,10 +4618,36 @@ void mesh_bake_upload(const MeshBakeSetup& S, tcloth::BakeGpu& G, cudaStream_t s
   tcloth::k_bone_tile_spheres<<<(G.ntiles + 127) / 128, 128, 0, st>>>(G.ntiles, G.tile_first.p, G.tile_cnt.p, G.sph.p,
                                                                        G.tsph.p);
 }
-tcloth::MeshBakeParams mesh_bake_params(const MeshBakeSetup& S, uint32_t ntri) {
-  return tcloth::MeshBakeParams{{S.lo[0], S.lo[1], S.lo[2]}, {S.hi[0], S.hi[1], S.hi[2]}, S.dim[0], S.dim[1], S.dim[2],
-                                ntri};
-}
+// triangles on the device, in Morton order with the spheres of their runs
+struct MeshBakeGpu {
+  uint32_t nt = 0;
+  tcloth::DBuf<BakeTri> tris;
+  tcloth::DBuf<float4> sph, psph, s8, s64, s512;
+  tcloth::DBuf<uint32_t> key;  // codes and indices, before and after the sort
+  tcloth::DBuf<unsigned char> tmp;
+  tcloth::MeshTree tree{};
+  void upload(const MeshBakeSetup& S, cudaStream_t st) {
+    nt = uint32_t(S.tris.size());
+    const uint32_t n8 = (nt + 7) / 8, n64 = (n8 + 7) / 8, n512 = (n64 + 7) / 8;
+    auto blocks = [](uint32_t c) { return (c + 127) / 128; };
+    tris.upload(S.tris, st);
+    sph.alloc(nt); psph.alloc(nt); s8.alloc(n8); s64.alloc(n64); s512.alloc(n512);
+    key.alloc(4 * size_t(nt));
+    uint32_t *c0 = key.p, *c1 = c0 + nt, *i0 = c1 + nt, *i1 = i0 + nt;
+    tcloth::k_mesh_codes<<<blocks(nt), 128, 0, st>>>(nt, tris.p, mesh_bake_params(S, nt), c0, i0);
+    size_t bytes = 0;
+    TC_CK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, c0, c1, i0, i1, int(nt), 0, 30, st));
+    tmp.alloc(bytes);
+    TC_CK(cub::DeviceRadixSort::SortPairs(tmp.p, bytes, c0, c1, i0, i1, int(nt), 0, 30, st));
+    tcloth::k_bone_tri_spheres<<<blocks(nt), 128, 0, st>>>(nt, tris.p, sph.p);
+    tcloth::k_bake_perm_spheres<<<blocks(nt), 128, 0, st>>>(nt, i1, sph.p, psph.p);
+    tcloth::k_group8_spheres<<<blocks(n8), 128, 0, st>>>(nt, psph.p, s8.p);
+    tcloth::k_group8_spheres<<<blocks(n64), 128, 0, st>>>(n8, s8.p, s64.p);
+    tcloth::k_group8_spheres<<<blocks(n512), 128, 0, st>>>(n64, s64.p, s512.p);
+    TC_CK(cudaGetLastError());
+    tree = tcloth::MeshTree{nt, i1, psph.p, s8.p, s64.p, s512.p};
+  }
+};
 uint32_t brick_blocks(const uint32_t dim[3]) {
   return ((dim[0] + 7) / 8) * ((dim[1] + 7) / 8) * ((dim[2] + 3) / 4);
 }
@@ -4645,13 +4699,12 @@ tc_status tc_bake_mesh_sdf(const float* mesh_verts, uint32_t nv, const int32_t* 
     R->w = S.dim[0]; R->h = S.dim[1]; R->d = S.dim[2];
     R->infos = S.infos;
     OwnStream os(device);
-    tcloth::BakeGpu G;
-    mesh_bake_upload(S, G, os.s);
+    MeshBakeGpu G;
+    G.upload(S, os.s);
     const size_t nvox = size_t(S.dim[0]) * S.dim[1] * S.dim[2];
     tcloth::DBuf<uint32_t> vox;
     vox.alloc(nvox);
-    tcloth::k_mesh_bake<<<brick_blocks(S.dim), 256, 0, os.s>>>(mesh_bake_params(S, G.nt), G.tris.p, G.sph.p, G.tsph.p,
-                                                                vox.p);
+    tcloth::k_mesh_bake<<<brick_blocks(S.dim), 256, 0, os.s>>>(mesh_bake_params(S, G.nt), G.tris.p, G.tree, vox.p);
     R->texels.resize(nvox);
     TC_CK(cudaMemcpyAsync(R->texels.data(), vox.p, nvox * 4, cudaMemcpyDeviceToHost, os.s));
     TC_CK(cudaStreamSynchronize(os.s));
