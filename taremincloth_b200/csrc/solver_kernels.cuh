@@ -501,12 +501,24 @@ struct ColliderArgs {
   BoneSdfArgs bone;       // bone SDF colliders (nbones == 0: off)
 };
 
-// Conservative skip test for a group of triangles: true only when every
-// member triangle would fail its own test seg_point_d2 > (1.5 r + th)^2.
-__device__ __forceinline__ bool group_far(V3 a, V3 b, float4 g, float th) {
-  float R = g.w + th;
-  float d2 = seg_point_d2(a, b, mk(g));
-  return d2 > R * R * 1.0004f + 1e-12f;
+// The ball around a vertex's motion segment, for the mesh collider's skip
+// tests: centre, radius widened by a relative 1e-3 and by 1e-6 of the
+// coordinates, which covers the rounding of these tests and of
+// segment-to-centre distances.  seg_point_d2 costs a division; most triangles
+// and groups are ruled out without it.
+struct SegBall {
+  V3 c;
+  float h;
+};
+__device__ __forceinline__ SegBall seg_ball(V3 a, V3 b) {
+  const V3 c = (a + b) * 0.5f;
+  return SegBall{c, length(b - a) * 0.5005f + 1e-6f * (fabsf(c.x) + fabsf(c.y) + fabsf(c.z)) + 1e-6f};
+}
+// true only when the segment is farther than r from the point
+__device__ __forceinline__ bool ball_far(const SegBall& s, float4 g, float r) {
+  const V3 d = s.c - mk(g);
+  const float R = r * 1.001f + s.h;
+  return dot(d, d) > R * R;
 }
 
 // shaders/collision.wgsl:378-652 (cluster culling off, the reference
@@ -568,20 +580,22 @@ __device__ __forceinline__ void collide_vertex_m(uint32_t i, const M& m, const C
     st.bpos = p;
     st.bn = mk(0.f, 0.f, 0.f);
     const uint32_t ng256 = (ca.ntris + 255u) / 256u, ng4096 = (ca.ntris + 4095u) / 4096u;
+    SegBall ball = seg_ball(xpos, p);
     for (uint32_t g4 = 0; g4 < ng4096; ++g4) {
-      if (group_far(xpos, p, ca.cl4096[g4], th)) continue;
+      if (ball_far(ball, ca.cl4096[g4], ca.cl4096[g4].w + th)) continue;
       const uint32_t g_end = min((g4 + 1u) * 16u, ng256);
       for (uint32_t g = g4 * 16u; g < g_end; ++g) {
-        if (group_far(xpos, p, ca.cl256[g], th)) continue;
+        if (ball_far(ball, ca.cl256[g], ca.cl256[g].w + th)) continue;
         const uint32_t c_end = min((g + 1u) * 16u, (ca.ntris + 15u) / 16u);
         for (uint32_t cgi = g * 16u; cgi < c_end; ++cgi) {
-          if (group_far(xpos, p, ca.cl16[cgi], th)) continue;
+          if (ball_far(ball, ca.cl16[cgi], ca.cl16[cgi].w + th)) continue;
           const uint32_t t_end = min((cgi + 1u) * 16u, ca.ntris);
           for (uint32_t t = cgi * 16u; t < t_end; ++t) {
             const float4 b = ca.bounds[t];
             const float r = b.w * 1.5f + th;
-            if (seg_point_d2(xpos, p, mk(b)) > r * r) continue;
+            if (ball_far(ball, b, r) || seg_point_d2(xpos, p, mk(b)) > r * r) continue;
             mesh_triangle(ca.tris[t], th, xpos, p, xn, dt, pinit, ca.recovery, st);
+            ball = seg_ball(xpos, p);  // a contact moves p
           }
         }
       }
