@@ -8,6 +8,7 @@
 // counting sort (atomic scatter, shaders/spatial_grid_sort.wgsl:182-194), is
 // made canonical here: each bucket is sorted by ascending element index.
 #pragma once
+#include "solver_kernels.cuh"
 #include "vmath.cuh"
 
 namespace tcloth {
@@ -159,18 +160,21 @@ __device__ __forceinline__ TwoHop stage_two_hop(const uint32_t* th_off, const ui
 __device__ __forceinline__ uint32_t layer_of(const float4* v4, uint32_t i) { return __float_as_uint(v4[i].w); }
 
 // Star boxes and star-entry records for the vertex-triangle pass (see
-// SCArgs::sbox, st_lo): one thread per vertex over its star pairs.
+// SCArgs::sbox, st_lo), and with nrm the area-weighted normals (k_normals, which
+// reads the same positions): one thread per vertex over its star pairs.
 __global__ void k_star_box(uint32_t n, const uint32_t* __restrict__ star_off, const uint2* __restrict__ star_idx,
                            const float4* __restrict__ x4, const float4* __restrict__ p4, float4* __restrict__ sbox,
-                           float4* __restrict__ st_lo, float4* __restrict__ st_hi, float* __restrict__ st_mz) {
+                           float4* __restrict__ st_lo, float4* __restrict__ st_hi, float* __restrict__ st_mz,
+                           float4* __restrict__ nrm) {
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
   const V3 pj = mk(p4[j]), pjo = mk(x4[j]);
-  V3 lo = pj, hi = pj, mlo = pj - pjo, mhi = mlo;
+  V3 lo = pj, hi = pj, mlo = pj - pjo, mhi = mlo, ns = mk(0.f, 0.f, 0.f);
   for (uint32_t k = star_off[j]; k < star_off[j + 1]; ++k) {
     const uint2 pr = star_idx[k];
     const V3 a = mk(p4[pr.x]), b = mk(p4[pr.y]);
-    const V3 ma = a - mk(x4[pr.x]), mb = b - mk(x4[pr.y]);
+    const V3 ao = mk(x4[pr.x]), bo = mk(x4[pr.y]), ma = a - ao, mb = b - bo;
+    ns = ns + cross(ao - pjo, bo - pjo);
     lo = vmin(lo, vmin(a, b));
     hi = vmax(hi, vmax(a, b));
     mlo = vmin(mlo, vmin(ma, mb));
@@ -184,6 +188,11 @@ __global__ void k_star_box(uint32_t n, const uint32_t* __restrict__ star_off, co
   sbox[3 * size_t(j)] = make_float4(lo.x, lo.y, lo.z, mlo.x);
   sbox[3 * size_t(j) + 1] = make_float4(hi.x, hi.y, hi.z, mlo.y);
   sbox[3 * size_t(j) + 2] = make_float4(mhi.x, mhi.y, mhi.z, mlo.z);
+  if (nrm) {
+    const float l = length(ns);
+    const V3 r = l > kEps ? ns / l : mk(0.f, 0.f, 0.f);
+    nrm[j] = make_float4(r.x, r.y, r.z, 0.f);
+  }
 }
 
 // ---------------- normals: shaders/compute_normals.wgsl:25-58
@@ -288,6 +297,35 @@ __global__ void __launch_bounds__(1024) k_scan_finish(uint32_t table, uint32_t n
     starts[i] += tile_off[i >> 10];
 }
 
+// The same scan in one launch: a block sums the counts before its 1,024-entry
+// tile itself (at most 63 tiles, from L2) instead of waiting for another
+// launch's tile totals.
+__global__ void __launch_bounds__(1024) k_hash_scan(uint32_t table, const uint32_t* __restrict__ counts,
+                                                    uint32_t* __restrict__ starts) {
+  __shared__ uint32_t warp_tot[32], before[32];
+  const uint32_t i = blockIdx.x * 1024u + threadIdx.x;
+  uint32_t b = 0;
+  for (uint32_t k = threadIdx.x; k < blockIdx.x * 1024u; k += 1024u) b += counts[k];
+  b = __reduce_add_sync(0xffffffffu, b);
+  if ((threadIdx.x & 31u) == 0) before[threadIdx.x >> 5] = b;
+  const uint32_t c = i < table ? counts[i] : 0u;
+  uint32_t total;
+  const uint32_t incl = block_incl_scan_1024(c, warp_tot, total);  // (synchronises the block)
+  const uint32_t base = __reduce_add_sync(0xffffffffu, before[threadIdx.x & 31u]);
+  if (i < table) starts[i] = base + incl - c;
+  if (i == table - 1u) starts[table] = base + incl;
+}
+// Scatter that takes the counts down again: they are zero for the next build
+// without a clear, and no cursors are needed (the in-bucket order is made
+// canonical afterwards).
+__global__ void k_hash_place(uint32_t cnt, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ starts,
+                             uint32_t* __restrict__ counts, uint32_t* __restrict__ sorted) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= cnt) return;
+  const uint32_t h = keys[i];
+  sorted[starts[h] + atomicSub(&counts[h], 1u) - 1u] = i;
+}
+
 __global__ void k_hash_scatter(uint32_t cnt, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ starts,
                                uint32_t* __restrict__ cursor, uint32_t* __restrict__ sorted) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -361,25 +399,19 @@ __global__ void k_hash_sort_buckets(uint32_t table, const uint32_t* __restrict__
   }
 }
 
-// The same canonical order (each bucket ascending), one warp per bucket: up
-// to 64 entries are sorted in registers by a bitonic network (two per lane,
-// padding 0xFFFFFFFF, which no index reaches); up to kSortRankCap entries by
-// rank in shared memory; longer buckets fall back to the serial insertion
-// sort on lane 0.  Blocks of 8 warps.
+// The same canonical order (each bucket ascending), one warp per 32 buckets,
+// most of which hold nothing to sort (a warp per bucket spent 22 us on 65,536
+// buckets, 10 us of it on empty ones): a bucket of up to 64 entries is sorted in
+// registers by a bitonic network (two per lane, padding 0xFFFFFFFF, which no
+// index reaches); up to kSortRankCap entries by rank in shared memory; longer
+// buckets fall back to the serial insertion sort on lane 0.  Blocks of 4 warps.
 constexpr uint32_t kSortRankCap = 1024;
-__global__ void __launch_bounds__(256) k_hash_sort_buckets_warp(uint32_t table, const uint32_t* __restrict__ starts,
-                                                                uint32_t* __restrict__ sorted) {
-  __shared__ uint32_t sh_sort[8][kSortRankCap];
-  const uint32_t h = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const uint32_t lane = threadIdx.x & 31u;
-  if (h >= table) return;  // whole warp
-  const uint32_t b = starts[h], e = starts[h + 1];
+__device__ __forceinline__ void sort_bucket(uint32_t b, uint32_t e, uint32_t lane, uint32_t* buf,
+                                            uint32_t* __restrict__ sorted) {
   const uint32_t n = e - b;
-  if (n < 2) return;
   if (n > 64 && n <= kSortRankCap) {
     // rank sort in shared memory: the entries are distinct indices, so the
     // rank of v (the number of smaller entries) is its sorted position
-    uint32_t* buf = sh_sort[threadIdx.x >> 5];
     for (uint32_t i = lane; i < n; i += 32u) buf[i] = sorted[b + i];
     __syncwarp();
     for (uint32_t i = lane; i < n; i += 32u) {
@@ -402,7 +434,8 @@ __global__ void __launch_bounds__(256) k_hash_sort_buckets_warp(uint32_t table, 
   }
   uint32_t a0 = lane < n ? sorted[b + lane] : 0xFFFFFFFFu;
   uint32_t a1 = lane + 32u < n ? sorted[b + lane + 32u] : 0xFFFFFFFFu;
-  const uint32_t kmax = n > 32 ? 64u : 32u;
+  // (entries past n are padding: networks of 8, 16, 32 or 64)
+  const uint32_t kmax = n > 32 ? 64u : n > 16 ? 32u : n > 8 ? 16u : 8u;
   for (uint32_t k = 2; k <= kmax; k <<= 1) {
     for (uint32_t j = k >> 1; j > 0; j >>= 1) {
       if (j == 32u) {  // partners lane and lane + 32 live in one lane
@@ -422,6 +455,22 @@ __global__ void __launch_bounds__(256) k_hash_sort_buckets_warp(uint32_t table, 
   }
   if (lane < n) sorted[b + lane] = a0;
   if (lane + 32u < n) sorted[b + lane + 32u] = a1;
+}
+__global__ void __launch_bounds__(128) k_hash_sort_buckets_warp(uint32_t table, const uint32_t* __restrict__ starts,
+                                                                uint32_t* __restrict__ sorted) {
+  __shared__ uint32_t sh_sort[4][kSortRankCap];
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t h = (blockIdx.x * 4u + (threadIdx.x >> 5)) * 32u + lane;
+  uint32_t b = 0, e = 0;
+  if (h < table) {
+    b = starts[h];
+    e = starts[h + 1];
+  }
+  for (uint32_t todo = __ballot_sync(0xffffffffu, e - b >= 2u); todo; todo &= todo - 1u) {
+    const int k = __ffs(todo) - 1;
+    sort_bucket(__shfl_sync(0xffffffffu, b, k), __shfl_sync(0xffffffffu, e, k), lane, sh_sort[threadIdx.x >> 5], sorted);
+    __syncwarp();
+  }
 }
 
 // ---------------- accumulation helpers (shaders/self_collision.wgsl:77-118)
@@ -2250,9 +2299,11 @@ __global__ void __launch_bounds__(256) k_edge_collision(EdgeColArgs a) {
 }
 
 // ---------------- sc_apply: shaders/self_collision_apply.wgsl:57-177
-__global__ void k_apply(uint32_t n, const float4* __restrict__ x4, float4* __restrict__ p4,
+// kUpdate: followed by the substep's velocity update (update_vertex_m).
+template <bool kUpdate>
+__global__ void k_apply(uint32_t n, float4* __restrict__ x4, float4* __restrict__ p4,
                         const float* __restrict__ local_len, int32_t* __restrict__ acc, float relief, int enable_relief,
-                        float max_disp_ratio) {
+                        float max_disp_ratio, float4* __restrict__ v4, float dt_sub) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int4* a4 = reinterpret_cast<int4*>(acc + (size_t)i * A_N);
@@ -2289,6 +2340,7 @@ __global__ void k_apply(uint32_t n, const float4* __restrict__ x4, float4* __res
     p.x += fd.x; p.y += fd.y; p.z += fd.z;
     p4[i] = p;
   }
+  if (kUpdate) update_vertex<false>(i, x4, p4, v4, dt_sub);
 }
 
 }  // namespace tcloth

@@ -644,9 +644,9 @@ struct Sim {
   DBuf<float4> dist_par, bend_par;
   DBuf<uint4> bend_ids;
   DBuf<uint32_t> adj_off, adj_idx, th_off, th_idx, star_off, edge_bits;
-  DBuf<uint32_t> keys, counts, cursor, cs, srt, ekeys, ecs, esrt, ecounts, ecursor, etile_sum;
+  DBuf<uint32_t> keys, counts, cs, srt, ekeys, ecs, esrt, ecounts;
   cudaStream_t st2 = nullptr;  // edge side of self-collision
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_nrm = nullptr;
   DBuf<float4> nrm;
   DBuf<int32_t> acc;
   DBuf<int4> vcell, ecell;
@@ -655,7 +655,6 @@ struct Sim {
   DBuf<float> mlen;
   DBuf<float4> eamin, eamax;
   DBuf<float4> vs_p, vs_q, es_lo, es_hi;
-  DBuf<uint32_t> tile_sum;
   DBuf<int4> vs_c, es_c;
   DBuf<uint2> es_v, ccd_q, ee_q;
   DBuf<uint32_t> ccd_n;  // [0] deferred CCD pairs, [1 + g] listed E-E pairs of segment g
@@ -734,9 +733,17 @@ struct Sim {
                   kColEdgeTable, edge_mscale, edge_moff, acc.p};
     timed("edge_collision", [&] { k_edge_collision<<<grid(ne, 256), 256, 0, st>>>(a); });
     timed("edge_apply", [&] {
-      k_apply<<<grid(n, 256), 256, 0, st>>>(n, x4.p, p4.p, local_len.p, acc.p, relief, enable_relief ? 1 : 0,
-                                             max_disp_ratio);
+      launch_apply(nullptr);
     });
+  }
+  // the apply pass, with dts the velocity update of a substep of *dts too
+  void launch_apply(const float* dts) {
+    if (dts)
+      k_apply<true><<<grid(n, 256), 256, 0, st>>>(n, x4.p, p4.p, local_len.p, acc.p, relief, enable_relief ? 1 : 0,
+                                                   max_disp_ratio, v4.p, *dts);
+    else
+      k_apply<false><<<grid(n, 256), 256, 0, st>>>(n, x4.p, p4.p, local_len.p, acc.p, relief, enable_relief ? 1 : 0,
+                                                    max_disp_ratio, v4.p, 0.f);
   }
   DBuf<Prim> prims;
   DBuf<MeshTri> tris;
@@ -964,6 +971,7 @@ struct Sim {
     for (auto e : ev_pool) cudaEventDestroy(e);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
+    if (ev_nrm) cudaEventDestroy(ev_nrm);
     if (st2) cudaStreamDestroy(st2);
     if (st) cudaStreamDestroy(st);
     if (h_err) cudaFreeHost(h_err);
@@ -1214,12 +1222,16 @@ struct Sim {
     edges.upload(reinterpret_cast<const uint2*>(m.edges.data()), ne, st);
     edge_bits.upload(m.edge_bits, st);
     const size_t T = m.table;
-    keys.alloc(n); counts.alloc(T + 1); cursor.alloc(T + 1); cs.alloc(T + 1); srt.alloc(n);
+    keys.alloc(n); counts.alloc(T + 1); cs.alloc(T + 1); srt.alloc(n);
     ekeys.alloc(ne); ecs.alloc(T + 1); esrt.alloc(ne);
-    ecounts.alloc(T + 1); ecursor.alloc(T + 1); etile_sum.alloc(64);
+    ecounts.alloc(T + 1);
+    // zero between builds: every build takes its counts down again
+    TC_CK(cudaMemsetAsync(counts.p, 0, (T + 1) * sizeof(uint32_t), st));
+    TC_CK(cudaMemsetAsync(ecounts.p, 0, (T + 1) * sizeof(uint32_t), st));
     TC_CK(cudaStreamCreateWithFlags(&st2, cudaStreamNonBlocking));
     TC_CK(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
     TC_CK(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
+    TC_CK(cudaEventCreateWithFlags(&ev_nrm, cudaEventDisableTiming));
     nrm.alloc(n);
     acc.alloc(size_t(n) * A_N);
     vcell.alloc(n); mlen.alloc(n); sbox.alloc(3 * size_t(n));
@@ -1227,7 +1239,7 @@ struct Sim {
     ecell.alloc(ne); eamin.alloc(ne); eamax.alloc(ne);
     ccd_q.alloc(size_t(ne) * 8 + 1024); ccd_n.alloc(1 + tcloth::kEeSeg);
     ee_q.alloc(size_t(ne) * 24 + 1024);
-    vs_p.alloc(n); vs_q.alloc(n); vs_c.alloc(n); tile_sum.alloc(64); es_c.alloc(ne); es_v.alloc(ne); es_lo.alloc(ne); es_hi.alloc(ne);
+    vs_p.alloc(n); vs_q.alloc(n); vs_c.alloc(n); es_c.alloc(ne); es_v.alloc(ne); es_lo.alloc(ne); es_hi.alloc(ne);
     TC_CK(cudaMemsetAsync(acc.p, 0, size_t(n) * A_N * sizeof(int32_t), st));
     TC_CK(cudaMemsetAsync(nrm.p, 0, size_t(n) * sizeof(float4), st));
     res_sum.alloc(m.dist_cnt.size() + m.bend_cnt.size() + 1);
@@ -1480,19 +1492,13 @@ struct Sim {
     uint32_t* start = which == 0 ? cs.p : ecs.p;
     uint32_t* sorted = which == 0 ? srt.p : esrt.p;
     uint32_t* cnts = which == 0 ? counts.p : ecounts.p;
-    uint32_t* curs = which == 0 ? cursor.p : ecursor.p;
-    uint32_t* tsum = which == 0 ? tile_sum.p : etile_sum.p;
-    TC_CK(cudaMemsetAsync(cnts, 0, (T + 1) * sizeof(uint32_t), ss));
-    TC_CK(cudaMemsetAsync(curs, 0, (T + 1) * sizeof(uint32_t), ss));
     timed(which == 0 ? "hash_vertices" : "hash_edges", [&] {
       if (cnt)
         k_hash_count<<<grid(cnt, 256), 256, 0, ss>>>(cnt, which, x4.p, p4.p, edges.p, m.cell, T, k, cnts,
                                                       which == 0 ? vcell.p : ecell.p, mlen.p, eamin.p, eamax.p);
-      const uint32_t ntiles = (T + 1023) / 1024;
-      k_scan_blocks<<<ntiles, 1024, 0, ss>>>(T, cnts, start, tsum);
-      k_scan_finish<<<ntiles, 1024, 0, ss>>>(T, ntiles, tsum, start);
-      if (cnt) k_hash_scatter<<<grid(cnt, 256), 256, 0, ss>>>(cnt, k, start, curs, sorted);
-      k_hash_sort_buckets_warp<<<grid(T, 8), 256, 0, ss>>>(T, start, sorted);
+      k_hash_scan<<<(T + 1023) / 1024, 1024, 0, ss>>>(T, cnts, start);
+      if (cnt) k_hash_place<<<grid(cnt, 256), 256, 0, ss>>>(cnt, k, start, cnts, sorted);
+      k_hash_sort_buckets_warp<<<grid(T, 128), 128, 0, ss>>>(T, start, sorted);
       if (cnt && which == 0)
         k_gather_vertices<<<grid(cnt, 256), 256, 0, ss>>>(cnt, sorted, x4.p, p4.p, v4.p, local_len.p, mlen.p, vcell.p,
                                                            vs_p.p, vs_c.p, vs_q.p);
@@ -1527,15 +1533,19 @@ struct Sim {
     else if (ne < 50000u) launch_ee_v<4>(a, ss);
     else launch_ee_v<8>(a, ss);
   }
-  void encode_ee(const SCArgs& a, cudaStream_t ss) {
+  // normals: null, or the event after which they are there (recorded on another stream)
+  void encode_ee(const SCArgs& a, cudaStream_t ss, cudaEvent_t normals = nullptr) {
     timed("sc_solve_ee", [&] {
       TC_CK(cudaMemsetAsync(ccd_n.p, 0, (1 + tcloth::kEeSeg) * sizeof(uint32_t), ss));
+      const bool listed = !ee_grouped && a.ee_cap;
+      if (normals && !listed) TC_CK(cudaStreamWaitEvent(ss, normals, 0));
       if (ee_grouped) {
         k_ee_grouped<<<grid(ne, 32 * tcloth::kEeWarps), 32 * tcloth::kEeWarps, 0, ss>>>(a);
       } else {
         if (a.ee_cap)
           launch_ee_cluster(a, ss);
         else k_ee<<<grid(ne, 8), 256, 0, ss>>>(a);
+        if (normals && listed) TC_CK(cudaStreamWaitEvent(ss, normals, 0));
         if (a.ee_cap) k_ee_pairs<<<tcloth::kEeSeg * tcloth::kEePairBlocks, 256, 0, ss>>>(a);
       }
     });
@@ -1561,7 +1571,7 @@ struct Sim {
   // (a warp per block: the scans' lengths differ, and the 2,500 warps of 80,000
   // vertices are 1.4 waves; 128 threads: 12.4 ms a frame, 64: 12.1, 32: 11.8)
   static constexpr unsigned kPairBlock = 32;
-  void encode_pair_self_collision(bool run_ee, bool rebuild, float dt) {
+  void encode_pair_self_collision(bool run_ee, bool rebuild, float dt, const float* update_dts) {
     SCArgs a = sc_args();
     const PairArgs p = pair_args(dt);
     if (a.untangle) timed("sc_normals", [&] { k_normals<<<grid(n, 256), 256, 0, st>>>(n, x4.p, star_off.p, star_idx.p, nrm.p); });
@@ -1587,41 +1597,46 @@ struct Sim {
     timed("pair_vt", [&] { k_pair_vt<<<grid(vts, 128), 128, 0, st>>>(a, p, vts); });
     if (run_ee) timed("pair_ee", [&] { k_pair_ee<<<grid(ees, 128), 128, 0, st>>>(a, p, ees); });
     if (a.untangle) timed("sc_untangle", [&] { k_untangle<<<grid(n, 128), 128, 0, st>>>(a); });
-    timed("sc_apply", [&] {
-      k_apply<<<grid(n, 256), 256, 0, st>>>(n, x4.p, p4.p, local_len.p, acc.p, relief, enable_relief ? 1 : 0,
-                                             max_disp_ratio);
-    });
+    timed("sc_apply", [&] { launch_apply(update_dts); });
   }
 
-  void encode_self_collision(bool run_ee, uint32_t s, uint32_t substeps, float dt) {
+  // update_dts: see launch_apply
+  void encode_self_collision(bool run_ee, uint32_t s, uint32_t substeps, float dt, const float* update_dts) {
     if (rec_pairs) TC_CK(cudaMemsetAsync(rec_n.p, 0, 2 * sizeof(uint32_t), st));
     const bool force_direct = pair_cache && pair_final_fallback && s + 1 == substeps;
     if (pair_cache && !force_direct) {
-      encode_pair_self_collision(run_ee, s == 0, dt);
+      encode_pair_self_collision(run_ee, s == 0, dt, update_dts);
       return;
     }
     SCArgs a = sc_args();
-    if (a.untangle) timed("sc_normals", [&] { k_normals<<<grid(n, 256), 256, 0, st>>>(n, x4.p, star_off.p, star_idx.p, nrm.p); });
     const bool edges_on = run_ee && ne > 0;
     const bool fork = edges_on && !profiling;
+    // star boxes and normals first: of the edge side only the contact work
+    // needs the normals
+    auto stars = [&] {
+      timed("sc_star_box", [&] {
+        k_star_box<<<grid(n, 256), 256, 0, st>>>(n, star_off.p, star_idx.p, x4.p, p4.p, sbox.p, st_lo.p, st_hi.p,
+                                                 st_mz.p, a.untangle ? nrm.p : nullptr);
+      });
+    };
     if (fork) {
       TC_CK(cudaEventRecord(ev_fork, st));
       TC_CK(cudaStreamWaitEvent(st2, ev_fork, 0));
+      stars();
+      TC_CK(cudaEventRecord(ev_nrm, st));
       encode_hash(1, st2);
-      encode_ee(a, st2);
+      encode_ee(a, st2, a.untangle ? ev_nrm : nullptr);
       TC_CK(cudaEventRecord(ev_join, st2));
+    } else {
+      stars();
     }
     encode_hash(0);
-    timed("sc_star_box", [&] { k_star_box<<<grid(n, 256), 256, 0, st>>>(n, star_off.p, star_idx.p, x4.p, p4.p, sbox.p, st_lo.p, st_hi.p, st_mz.p); });
     if (edges_on && !fork) encode_hash(1);
     timed("sc_solve", [&] { launch_sc_solve(a); });
     if (a.untangle) timed("sc_untangle", [&] { k_untangle<<<grid(n, 128), 128, 0, st>>>(a); });
     if (fork) TC_CK(cudaStreamWaitEvent(st, ev_join, 0));
     if (edges_on && !fork) encode_ee(a, st);
-    timed("sc_apply", [&] {
-      k_apply<<<grid(n, 256), 256, 0, st>>>(n, x4.p, p4.p, local_len.p, acc.p, relief, enable_relief ? 1 : 0,
-                                             max_disp_ratio);
-    });
+    timed("sc_apply", [&] { launch_apply(update_dts); });
   }
 
   ColliderArgs collider_args() {
@@ -2271,9 +2286,11 @@ struct Sim {
       }
       if (self_collision || edge_active()) {
         if (edge_active()) encode_edge_collision();
-        if (sc_due(s, substeps)) encode_self_collision(ee_due(s, substeps), s, substeps, dt);
+        const bool sc = sc_due(s, substeps);
+        if (sc) encode_self_collision(ee_due(s, substeps), s, substeps, dt, nsw ? nullptr : &sp.dt);
         if (nsw) timed("final_sewing", [&] { launch_sewing(sp.dt); });
-        timed("update_vel", [&] { launch_k(k_update_vel, grid(n, 256), 256, n, x4.p, p4.p, v4.p, sp.dt); });
+        if (!sc || nsw)
+          timed("update_vel", [&] { launch_k(k_update_vel, grid(n, 256), 256, n, x4.p, p4.p, v4.p, sp.dt); });
       } else if (colors) {
         if (nsw) timed("final_sewing", [&] { launch_sewing(sp.dt); });
         timed("update_vel", [&] { launch_k(k_update_vel, grid(n, 256), 256, n, x4.p, p4.p, v4.p, sp.dt); });
@@ -2461,9 +2478,10 @@ struct Sim {
         for (uint32_t s = 0; s < substeps; ++s) {
           launch_solver(solver_args(sp, 1, use_coupled, false));
           if (edge_active()) encode_edge_collision();
-          if (sc_due(s, substeps)) encode_self_collision(ee_due(s, substeps), s, substeps, dt);
+          const bool sc = sc_due(s, substeps);
+          if (sc) encode_self_collision(ee_due(s, substeps), s, substeps, dt, nsw ? nullptr : &sp.dt);
           launch_sewing(sp.dt);  // final sewing (dispatch.rs:323-337)
-          k_update_vel<<<grid(n, 256), 256, 0, st>>>(n, x4.p, p4.p, v4.p, sp.dt);
+          if (!sc || nsw) k_update_vel<<<grid(n, 256), 256, 0, st>>>(n, x4.p, p4.p, v4.p, sp.dt);
         }
       }
       if (!use_resident()) TC_CK(cudaMemcpyAsync(h_err, &bar.p->err, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -2521,9 +2539,10 @@ struct Sim {
       if (hascol && !use_coupled) timed("collision", [&] { launch_collision(ca, dts); });
       if (npins) timed("pin", [&] { launch_k(k_pin, grid(npins, 128), 128, npins, pin_v.p, pin_t.p, x4.p, p4.p, dts); });
       if (edge_active()) encode_edge_collision();
-      if (sc_due(s, substeps)) encode_self_collision(ee_due(s, substeps), s, substeps, dt);
+      const bool sc = sc_due(s, substeps);
+      if (sc) encode_self_collision(ee_due(s, substeps), s, substeps, dt, nsw ? nullptr : &dts);
       if (nsw) timed("final_sewing", [&] { launch_sewing(dts); });
-      timed("update_vel", [&] { launch_k(k_update_vel, grid(n, 256), 256, n, x4.p, p4.p, v4.p, dts); });
+      if (!sc || nsw) timed("update_vel", [&] { launch_k(k_update_vel, grid(n, 256), 256, n, x4.p, p4.p, v4.p, dts); });
     }
     TC_CK(cudaGetLastError());
   }
