@@ -1432,6 +1432,96 @@ __device__ __forceinline__ bool outer_behind(const SCArgs& s, uint32_t la, uint3
   return allow && (dot(-dab, ni) < 0.0f);
 }
 
+// The continuous search of a moving edge pair
+// (shaders/self_collision_ee_direct.wgsl:404-470): nine samples of the squared
+// distance over the substep, one more where the pair's volume first changes
+// sign, then six ternary steps around the best.
+struct CcdMotion {
+  V3 a0o, a0, a1o, a1, b0o, b0, b1o, b1;
+  __device__ __forceinline__ float eval(float tau, float& so, float& to) const {
+    return seg_eval(a0o, a0, a1o, a1, b0o, b0, b1o, b1, tau, so, to);
+  }
+  __device__ __forceinline__ float vol(float tau) const { return seg_vol(a0o, a0, a1o, a1, b0o, b0, b1o, b1, tau); }
+};
+struct CcdBest {
+  float tau, d2, s, t;
+};
+__device__ __forceinline__ CcdBest ccd_search(const CcdMotion& m) {
+  float msd = 1e20f, btau = 0.0f, hs = 0.125f, ms = 0.f, mt = 0.f;
+  float pv = m.vol(0.0f);
+  float zc = -1.0f;
+  for (uint32_t k = 0; k <= 8u; ++k) {
+    const float tk = (float)k * 0.125f;
+    float es, et;
+    const float ed = m.eval(tk, es, et);
+    if (ed < msd) { msd = ed; btau = tk; ms = es; mt = et; }
+    if (k > 0u) {
+      const float vol = m.vol(tk);
+      if (pv * vol <= 0.0f && zc < 0.0f) zc = tk - 0.0625f;
+      pv = vol;
+    }
+  }
+  if (zc >= 0.0f) {
+    float es, et;
+    const float ed = m.eval(zc, es, et);
+    if (ed < msd) { msd = ed; btau = zc; hs = 0.0625f; ms = es; mt = et; }
+  }
+  float tlo = fmaxf(0.0f, btau - hs), thi = fminf(1.0f, btau + hs);
+  CcdBest r{btau, msd, ms, mt};
+  for (int it = 0; it < 6; ++it) {
+    const float m1 = tlo + (thi - tlo) * (1.0f / 3.0f);
+    const float mm2 = thi - (thi - tlo) * (1.0f / 3.0f);
+    float e1s, e1t, e2s, e2t;
+    const float e1 = m.eval(m1, e1s, e1t);
+    const float e2 = m.eval(mm2, e2s, e2t);
+    if (e1 < r.d2) r = CcdBest{m1, e1, e1s, e1t};
+    if (e2 < r.d2) r = CcdBest{mm2, e2, e2s, e2t};
+    if (e1 < e2) thi = mm2; else tlo = m1;
+  }
+  return r;
+}
+// The same by 8 lanes (all of the warp call it, groups of 8 with one pair
+// each): the samples one per lane, the two ends of a ternary step on the even
+// and odd lanes; 9 evaluations in a row instead of 22.  The same samples and
+// the same choices, so the same result, on every lane of the group.
+__device__ __forceinline__ CcdBest ccd_search8(const CcdMotion& m, uint32_t lane) {
+  const uint32_t r = lane & 7u, base = lane & 24u;
+  const float tk = (float)(r + 1u) * 0.125f;  // samples 1 to 8; sample 0 by every lane
+  float es, et, es0, et0;
+  const float ed0 = m.eval(0.0f, es0, et0), v0 = m.vol(0.0f);
+  const float ed = m.eval(tk, es, et), vk = m.vol(tk);
+  CcdBest best{0.0f, 1e20f, 0.f, 0.f};
+  if (ed0 < best.d2) best = CcdBest{0.0f, ed0, es0, et0};
+  float pv = v0, zc = -1.0f;
+#pragma unroll
+  for (uint32_t k = 0; k < 8u; ++k) {
+    const float d = __shfl_sync(0xffffffffu, ed, base + k), vol = __shfl_sync(0xffffffffu, vk, base + k);
+    const float qs = __shfl_sync(0xffffffffu, es, base + k), qt = __shfl_sync(0xffffffffu, et, base + k);
+    const float t = (float)(k + 1u) * 0.125f;
+    if (d < best.d2) best = CcdBest{t, d, qs, qt};
+    if (pv * vol <= 0.0f && zc < 0.0f) zc = t - 0.0625f;
+    pv = vol;
+  }
+  float hs = 0.125f;
+  if (zc >= 0.0f) {
+    const float d = m.eval(zc, es, et);
+    if (d < best.d2) { best = CcdBest{zc, d, es, et}; hs = 0.0625f; }
+  }
+  float tlo = fmaxf(0.0f, best.tau - hs), thi = fminf(1.0f, best.tau + hs);
+  for (int it = 0; it < 6; ++it) {
+    const float m1 = tlo + (thi - tlo) * (1.0f / 3.0f);
+    const float mm2 = thi - (thi - tlo) * (1.0f / 3.0f);
+    const float e = m.eval((r & 1u) ? mm2 : m1, es, et);
+    const float e1 = __shfl_sync(0xffffffffu, e, base), e2 = __shfl_sync(0xffffffffu, e, base + 1u);
+    const float s1 = __shfl_sync(0xffffffffu, es, base), s2 = __shfl_sync(0xffffffffu, es, base + 1u);
+    const float t1 = __shfl_sync(0xffffffffu, et, base), t2 = __shfl_sync(0xffffffffu, et, base + 1u);
+    if (e1 < best.d2) best = CcdBest{m1, e1, s1, t1};
+    if (e2 < best.d2) best = CcdBest{mm2, e2, s2, t2};
+    if (e1 < e2) thi = mm2; else tlo = m1;
+  }
+  return best;
+}
+
 struct EdgeCtx {
   uint32_t ei, u0, u1;
   float w_u0, w_u1;
@@ -1445,10 +1535,12 @@ struct EdgeCtx {
 
 // Contact work for one counted edge pair (shaders/self_collision_ee_direct.wgsl:356-774).
 // defer_ccd: the warp pass hands pairs that need the CCD search to the
-// one-thread-per-pair k_ee_ccd (inline when the queue is full).
+// one-thread-per-pair k_ee_ccd (inline when the queue is full).  pre: the
+// result of the pair's CCD search where it has run already.
 __device__ __forceinline__ void ee_pair(const SCArgs& s, const EdgeCtx& c, const TwoHop& th0, const TwoHop& th1,
                                         uint32_t eb, uint32_t j, uint32_t vj, const float4& qj, const float4& qvj,
-                                        const float4& xj, const float4& xvj, bool defer_ccd) {
+                                        const float4& xj, const float4& xvj, bool defer_ccd,
+                                        const CcdBest* pre = nullptr) {
   const uint32_t u0 = c.u0, u1 = c.u1;
   const float w_u0 = c.w_u0, w_u1 = c.w_u1;
   const bool apin = c.apin, bnda = c.bnda;
@@ -1489,37 +1581,9 @@ __device__ __forceinline__ void ee_pair(const SCArgs& s, const EdgeCtx& c, const
     }
   }
   if (run_ccd) {
-    float msd = 1e20f, btau = 0.0f, hs = 0.125f, ms = 0.f, mt = 0.f;
-    float pv = seg_vol(p_u0o, p_u0, p_u1o, p_u1, p_jo, p_j, p_vjo, p_vj, 0.0f);
-    float zc = -1.0f;
-    for (uint32_t k = 0; k <= 8u; ++k) {
-      const float tk = (float)k * 0.125f;
-      float es, et;
-      const float ed = seg_eval(p_u0o, p_u0, p_u1o, p_u1, p_jo, p_j, p_vjo, p_vj, tk, es, et);
-      if (ed < msd) { msd = ed; btau = tk; ms = es; mt = et; }
-      if (k > 0u) {
-        const float vol = seg_vol(p_u0o, p_u0, p_u1o, p_u1, p_jo, p_j, p_vjo, p_vj, tk);
-        if (pv * vol <= 0.0f && zc < 0.0f) zc = tk - 0.0625f;
-        pv = vol;
-      }
-    }
-    if (zc >= 0.0f) {
-      float es, et;
-      const float ed = seg_eval(p_u0o, p_u0, p_u1o, p_u1, p_jo, p_j, p_vjo, p_vj, zc, es, et);
-      if (ed < msd) { msd = ed; btau = zc; hs = 0.0625f; ms = es; mt = et; }
-    }
-    float tlo = fmaxf(0.0f, btau - hs), thi = fminf(1.0f, btau + hs);
-    float tstar = btau, dstar = msd, ss = ms, ts = mt;
-    for (int it = 0; it < 6; ++it) {
-      const float m1 = tlo + (thi - tlo) * (1.0f / 3.0f);
-      const float mm2 = thi - (thi - tlo) * (1.0f / 3.0f);
-      float e1s, e1t, e2s, e2t;
-      const float e1 = seg_eval(p_u0o, p_u0, p_u1o, p_u1, p_jo, p_j, p_vjo, p_vj, m1, e1s, e1t);
-      const float e2 = seg_eval(p_u0o, p_u0, p_u1o, p_u1, p_jo, p_j, p_vjo, p_vj, mm2, e2s, e2t);
-      if (e1 < dstar) { dstar = e1; tstar = m1; ss = e1s; ts = e1t; }
-      if (e2 < dstar) { dstar = e2; tstar = mm2; ss = e2s; ts = e2t; }
-      if (e1 < e2) thi = mm2; else tlo = m1;
-    }
+    const CcdMotion mo{p_u0o, p_u0, p_u1o, p_u1, p_jo, p_j, p_vjo, p_vj};
+    const CcdBest best = pre ? *pre : ccd_search(mo);
+    const float tstar = best.tau, dstar = best.d2, ss = best.s, ts = best.t;
     const float ets = mixf(thu0, thu1, ss) + mixf(thj, thvj, ts);
     if (dstar >= ets * ets) return;
     if (s.exclude_neighbors) {
@@ -1691,7 +1755,8 @@ __device__ __forceinline__ EdgeCtx edge_ctx(const SCArgs& s, uint32_t ei) {
 
 // Contact work for a listed (edge, edge) pair, with the two-hop lists of
 // the first edge's endpoints read from global memory.
-__device__ __forceinline__ void ee_listed_pair(const SCArgs& s, uint2 pr, bool defer_ccd) {
+__device__ __forceinline__ void ee_listed_pair(const SCArgs& s, uint2 pr, bool defer_ccd,
+                                               const CcdBest* pre = nullptr) {
   const EdgeCtx c = edge_ctx(s, pr.x);
   TwoHop th0, th1;
   th0.idx = s.th_idx + s.th_off[c.u0];
@@ -1701,7 +1766,7 @@ __device__ __forceinline__ void ee_listed_pair(const SCArgs& s, uint2 pr, bool d
   th1.rest = s.th_rest + s.th_off[c.u1];
   th1.n = s.th_off[c.u1 + 1] - s.th_off[c.u1];
   const uint2 ebv = s.edges[pr.y];
-  ee_pair(s, c, th0, th1, pr.y, ebv.x, ebv.y, s.p4[ebv.x], s.p4[ebv.y], s.x4[ebv.x], s.x4[ebv.y], defer_ccd);
+  ee_pair(s, c, th0, th1, pr.y, ebv.x, ebv.y, s.p4[ebv.x], s.p4[ebv.y], s.x4[ebv.x], s.x4[ebv.y], defer_ccd, pre);
 }
 
 // ee_listed_pair outside the caller's register allocation, for the rare
@@ -1724,12 +1789,25 @@ __global__ void __launch_bounds__(256, 4) k_ee_pairs(SCArgs s) {
   }
 }
 
-// Deferred CCD pairs, one thread each (the CCD search plus the discrete
-// fall-through of shaders/self_collision_ee_direct.wgsl:404-774).
+// Deferred CCD pairs (the CCD search plus the discrete fall-through of
+// shaders/self_collision_ee_direct.wgsl:404-774): one thread each when they
+// fill the launch, else 8 lanes each for the search, whose chain of evaluations
+// is then the launch's time.
 __global__ void __launch_bounds__(256, 3) k_ee_ccd(SCArgs s) {
   const uint32_t total = min(*s.ccd_n, s.ccd_cap);
-  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < total; q += gridDim.x * blockDim.x)
-    ee_listed_pair(s, s.ccd_q[q], false);
+  const uint32_t lane = threadIdx.x & 31u, width = total * 8u <= gridDim.x * blockDim.x ? 8u : 1u;
+  const uint32_t step = gridDim.x * blockDim.x / width;
+  const uint32_t first = (blockIdx.x * blockDim.x + threadIdx.x) / width;
+  for (uint32_t q = first; __any_sync(0xffffffffu, q < total); q += step) {
+    const bool on = q < total;
+    const uint2 pr = on ? s.ccd_q[q] : make_uint2(0u, 0u);
+    const uint2 a = on ? s.edges[pr.x] : make_uint2(0u, 0u), b = on ? s.edges[pr.y] : make_uint2(0u, 0u);
+    const CcdMotion m{mk(s.x4[a.x]), mk(s.p4[a.x]), mk(s.x4[a.y]), mk(s.p4[a.y]),
+                      mk(s.x4[b.x]), mk(s.p4[b.x]), mk(s.x4[b.y]), mk(s.p4[b.y])};
+    const CcdBest best = width == 8u ? ccd_search8(m, lane) : ccd_search(m);
+    if (on && (width == 1u || (lane & 7u) == 0u)) ee_listed_pair(s, pr, false, &best);
+    __syncwarp();
+  }
 }
 
 // One edge, searched by a warp in the reference's order: candidates of the 27
