@@ -2373,7 +2373,11 @@ struct Sim {
         const unsigned parts = persist_grid(bone_col);
         launch_k(k_ws_res_part, parts, 256, c);
         launch_k(k_ws_res_decide, 1, 32, c, uint32_t(parts));
-        for (uint32_t it = 0; it < kk; ++it) iteration(ws.gate.p);
+        // a threshold of +inf, which no residual exceeds, has no fallback to
+        // launch (28 kernels a substep on a batch of uneven cloths, 1 us each
+        // when the gate is shut)
+        const bool never = ws.res_ratio <= 0.f && std::isinf(ws.res_thresh) && ws.res_thresh > 0.f;
+        for (uint32_t it = 0; it < kk && !never; ++it) iteration(ws.gate.p);
       }
       k_ws_correction<<<grid(n, 256), 256, 0, st>>>(n, p4.p, ws.ppred.p, x4.p, local_len.p, ws.dprev.p, nullptr,
                                                     nullptr);
