@@ -306,6 +306,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_solver_resident(SolverArgs a
         else __syncthreads();
       }
     }
+    if (a.iters_only) {  // collision, pins and update are launches of their own
+      __syncthreads();
+      continue;
+    }
     // the rest of the substep touches only the CTA's own slice
     if (a.hascol && !a.coupled) own([&](uint32_t v, const ResOwn<kFull>& m) { collide_vertex_m<kBone>(v, m, a.ca, dts); });
     if (a.npins) {

@@ -78,13 +78,12 @@ struct SCArgs {
   uint2* ccd_q;
   uint32_t* ccd_n;
   uint32_t ccd_cap;
-  // (edge, edge) pairs counted by k_ee, worked one lane each by k_ee_pairs.
+  // (edge, edge) pairs counted by k_ee_cluster, worked one lane each by k_ee_pairs.
   // The list is split into kEeSeg segments of ee_cap / kEeSeg entries with a
-  // counter each (ee_n[kEeSeg]); block b of k_ee appends to segment
-  // b % kEeSeg, so that no one counter takes every warp's atomic.  A counter
+  // counter each (ee_n[kEeSeg]); block b of k_ee_cluster appends to
+  // segment b % kEeSeg, so that no one counter takes every warp's atomic.  A counter
   // may run past its segment's capacity (k_ee_pairs reads min(count, cap));
-  // the pairs past it are worked inside k_ee.  ee_cap = 0 keeps all of the
-  // contact work inside k_ee.
+  // the pairs past it are worked inside the filter.
   uint2* ee_q;
   uint32_t* ee_n;
   uint32_t ee_cap;
@@ -1773,7 +1772,7 @@ __device__ __forceinline__ void ee_listed_pair(const SCArgs& s, uint2 pr, bool d
 // pairs that do not fit the pair list.
 __device__ __noinline__ void ee_listed_pair_call(const SCArgs& s, uint2 pr) { ee_listed_pair(s, pr, true); }
 
-// Counted pairs listed by k_ee, one thread each: the CCD gate of
+// Counted pairs listed by k_ee_cluster, one thread each: the CCD gate of
 // shaders/self_collision_ee_direct.wgsl:361-403 and the discrete contact
 // from :632 on; pairs that need the CCD search go on to k_ee_ccd.
 // Grid: kEeSeg * kEePairBlocks blocks of 256 threads.

@@ -1138,12 +1138,30 @@ struct Sim {
       }
     const float ext = std::fmax(hi[0] - lo[0], std::fmax(hi[1] - lo[1], hi[2] - lo[2]));
     const float sc = ext > 0.f ? 1.f / ext : 0.f, inv[3] = {sc, sc, sc};
-    std::vector<uint64_t> key(cnt);
-    for (uint32_t i = 0; i < cnt; ++i)
-      key[i] = uint64_t(tcloth::morton3(at(i, 0), at(i, 1), at(i, 2), lo, inv)) << 32 | i;
-    std::sort(key.begin(), key.end());
-    std::vector<uint32_t> ord(cnt);
-    for (uint32_t i = 0; i < cnt; ++i) ord[i] = uint32_t(key[i]);
+    // stable radix sort of the 30-bit codes, 10 bits a pass
+    std::vector<uint32_t> key(cnt), ord(cnt), key2(cnt), ord2(cnt);
+    std::vector<uint32_t> cnts(3 * 1024, 0u);
+    for (uint32_t i = 0; i < cnt; ++i) {
+      key[i] = tcloth::morton3(at(i, 0), at(i, 1), at(i, 2), lo, inv);
+      ord[i] = i;
+      for (uint32_t d = 0; d < 3; ++d) ++cnts[d * 1024u + ((key[i] >> (10u * d)) & 1023u)];
+    }
+    for (uint32_t d = 0; d < 3; ++d) {
+      uint32_t* c = &cnts[d * 1024u];
+      uint32_t sum = 0;
+      for (uint32_t q = 0; q < 1024u; ++q) {
+        const uint32_t v = c[q];
+        c[q] = sum;
+        sum += v;
+      }
+      for (uint32_t i = 0; i < cnt; ++i) {
+        const uint32_t to = c[(key[i] >> (10u * d)) & 1023u]++;
+        key2[to] = key[i];
+        ord2[to] = ord[i];
+      }
+      key.swap(key2);
+      ord.swap(ord2);
+    }
     return ord;
   }
   void init(const MeshInput& in, int dev) {
@@ -1464,12 +1482,12 @@ struct Sim {
   // the collider pass's vertex order: Morton order of the initial positions
   DBuf<uint32_t> col_order, edge_order;
   float cell_ref = 0.f;  // the reference formula's hash cell (tc_set_hash_cell_size can override m.cell)
-  // E-E kernel: false = one warp per edge (k_ee), true = one lane per edge
+  // E-E kernel: false = k_ee_cluster or k_ee (below), true = one lane per edge
   // with per-cell candidate lists in shared memory (k_ee_grouped); same pairs
   // and results
   bool ee_grouped = false;
-  // k_ee lists its counted pairs for k_ee_pairs (one lane per pair) instead
-  // of working them in the edge's warp; same pairs and results.  The list
+  // k_ee_cluster lists the counted pairs for k_ee_pairs (one lane per pair);
+  // off: k_ee works them in the edge's warp; same pairs and results.  The list
   // holds ee_list_entries pairs (0: all of ee_q, 24 per edge + 1024).
   bool ee_list = true;
   size_t ee_list_entries = 0;
@@ -1754,6 +1772,7 @@ struct Sim {
     a.ndc = uint32_t(m.dist_cnt.size()); a.nbc = uint32_t(m.bend_cnt.size());
     a.hascol = has_colliders();
     a.coupled = use_coupled;
+    a.iters_only = false;
     a.ddamp = td != 0.f || cd != 0.f || sd != 0.f;
     a.bdamp = bd != 0.f;
     a.with_update = with_update;
@@ -2177,6 +2196,13 @@ struct Sim {
   // it is left to batches (one launch per frame) and to callers that ask for it.
   bool use_resident() const { return launch_auto && rs_ctas > 0; }
   bool use_persistent() const { return persistent && can_persist() && !(launch_auto && inst_vert_off.empty()); }
+  // A mesh collider worth several lanes per vertex leaves the resident launch,
+  // whose 16 CTAs have a thread per vertex: ms a frame of 10 substeps inside /
+  // outside, 3,200 vertices with self-collision over 80 triangles 1.21 / 1.16,
+  // 320: 1.36 / 1.20, 1,280: 1.52 / 1.22, 20,480: 3.38 / 1.41; without
+  // self-collision, where the frame is one launch inside, 0.43 / 0.44, 0.59 /
+  // 0.48, 0.76 / 0.52, 2.65 / 0.69.
+  bool split_collision(bool use_coupled) const { return use_resident() && !use_coupled && collision_lanes() > 1u; }
   void launch_solver(const SolverArgs& a) {
     if (use_resident()) launch_resident(a);
     else launch_persistent(a);
@@ -2451,8 +2477,27 @@ struct Sim {
   void launch_predict(const SubstepParams& sp) {
     launch_k(k_predict, grid(n, 256), 256, n, (const float4*)x4.p, p4.p, v4.p, sp, dlam.p, nd, blam.p, nb);
   }
+  // Lanes per vertex of the mesh-collider pass.  A thread per vertex walks the
+  // collider's spheres one after another, and up to 32,768 vertices are too few
+  // warps to hide that: 16 lanes test a run at once up to 8,192 vertices, 8
+  // above.  More vertices fill the chip and the lanes' common work on each
+  // contact costs more than the shorter walk gives; below 256 triangles there
+  // is little to walk.  us per pass at 1 / 8 / 16 lanes, (vertices, triangles):
+  // (3,200, 1,280) 67 / 31 / 22, (3,200, 20,480) 302 / 63 / 42,
+  // (9,800, 5,120) 89 / 42 / 30, (29,282, 5,120) 84 / 49 / 45 and 93 / 87 / 94
+  // with the cloth on the body, (29,282, 320) 37 / 32 / 36, (29,282, 80) 21 /
+  // 31 / 35, (64,800, 20,480) 121 / 110 / 114 and 164 / 278 / 329 on the body,
+  // (131,072, 20,480) 105 / 182 / 219.
+  uint32_t collision_lanes() const {
+    if (ntris < 256u || n > 32768u || bone.enabled) return 1u;
+    return n <= 8192u ? 16u : 8u;
+  }
   void launch_collision(const ColliderArgs& ca, float dts) {
     if (ca.bone.nbones > 0) launch_k(k_collision<true>, grid(n, 128), 128, n, x4.p, p4.p, ca, dts, col_order.p);
+    else if (collision_lanes() == 16u)
+      launch_k(k_collision_lanes<16>, grid(n * 16u, 128), 128, n, x4.p, p4.p, ca, dts, col_order.p);
+    else if (collision_lanes() == 8u)
+      launch_k(k_collision_lanes<8>, grid(n * 8u, 128), 128, n, x4.p, p4.p, ca, dts, col_order.p);
     else launch_k(k_collision<false>, grid(n, 128), 128, n, x4.p, p4.p, ca, dts, col_order.p);
   }
 
@@ -2476,11 +2521,18 @@ struct Sim {
     }
     if ((use_resident() || use_persistent()) && !profiling && !track_residual && !ws_recording()) {
       const SubstepParams sp = make_sp(dt / float(substeps));
-      if (!self_collision && !edge_active()) {
+      const bool split = split_collision(use_coupled);
+      if (!self_collision && !edge_active() && !split) {
         launch_solver(solver_args(sp, substeps, use_coupled, true));
       } else {
         for (uint32_t s = 0; s < substeps; ++s) {
-          launch_solver(solver_args(sp, 1, use_coupled, false));
+          SolverArgs a = solver_args(sp, 1, use_coupled, false);
+          a.iters_only = split;
+          launch_solver(a);
+          if (split) {
+            launch_collision(a.ca, sp.dt);
+            if (a.npins) launch_k(k_pin, grid(a.npins, 128), 128, a.npins, pin_v.p, pin_t.p, x4.p, p4.p, sp.dt);
+          }
           if (edge_active()) encode_edge_collision();
           const bool sc = sc_due(s, substeps);
           if (sc) encode_self_collision(ee_due(s, substeps), s, substeps, dt, nsw ? nullptr : &sp.dt);

@@ -521,20 +521,9 @@ __device__ __forceinline__ bool ball_far(const SegBall& s, float4 g, float r) {
   return dot(d, d) > R * R;
 }
 
-// shaders/collision.wgsl:378-652 (cluster culling off, the reference
-// default).  The triangle loop visits triangles in ascending (Morton) order
-// exactly like the reference; three levels of conservative bounding spheres
-// (4,096, 256 and 16 triangles, each enclosing its members' own test
-// spheres) skip runs of triangles none of which could pass the per-triangle
-// test, so the sequence of applied contacts is unchanged.
-template <bool kBone, class M>
-__device__ __forceinline__ void collide_vertex_m(uint32_t i, const M& m, const ColliderArgs& ca, float dt) {
-  float4 x = m.ldx(i);
-  if (x.w <= 0.0f) return;
-  float4 pr = m.ldp(i);
-  V3 p = mk(pr), pinit = p, xn = mk(x);
-  const V3 xpos = mk(x);
-  const float th = pr.w;
+// the sphere, capsule and plane colliders of one vertex, in order
+__device__ __forceinline__ void collide_prims(uint32_t i, const ColliderArgs& ca, float dt, float th, V3 pinit, V3& xn,
+                                              V3& p) {
   uint32_t kb = 0, ke = ca.nprims;
   if (ca.vinst) {
     const uint2 r = ca.inst_prims[ca.vinst[i]];
@@ -575,6 +564,23 @@ __device__ __forceinline__ void collide_vertex_m(uint32_t i, const M& m, const C
       if (dist < th) contact(p + pn * (th - dist), pn, fric, rest, dt, pinit, xn, p);
     }
   }
+}
+
+// shaders/collision.wgsl:378-652 (cluster culling off, the reference
+// default).  The triangle loop visits triangles in ascending (Morton) order
+// exactly like the reference; three levels of conservative bounding spheres
+// (4,096, 256 and 16 triangles, each enclosing its members' own test
+// spheres) skip runs of triangles none of which could pass the per-triangle
+// test, so the sequence of applied contacts is unchanged.
+template <bool kBone, class M>
+__device__ __forceinline__ void collide_vertex_m(uint32_t i, const M& m, const ColliderArgs& ca, float dt) {
+  float4 x = m.ldx(i);
+  if (x.w <= 0.0f) return;
+  float4 pr = m.ldp(i);
+  V3 p = mk(pr), pinit = p, xn = mk(x);
+  const V3 xpos = mk(x);
+  const float th = pr.w;
+  collide_prims(i, ca, dt, th, pinit, xn, p);
   if (ca.ntris > 0) {
     MeshState st;
     st.bpos = p;
@@ -635,6 +641,145 @@ __global__ void k_collision(uint32_t n, float4* __restrict__ x4, float4* __restr
   collide_vertex<false, kBone>(i, x4, p4, ca, dt);
 }
 
+// The same pass with kLanes lanes per vertex: the lanes test the 16 members of
+// a sphere's run at once and agree on a mask, then all of them work the first
+// member that is not skipped (the same values in every lane).  A mask holds
+// for the p it was tested with: once a contact moves p the rest is tested
+// again before it is used, so the triangles worked and their order are those of
+// collide_vertex_m.
+// Bound by the latency of the dependent sphere tests; the rule that chooses the
+// lanes has the figures.
+template <uint32_t kLanes>
+struct MeshWalk {
+  static constexpr uint32_t kEach = 16u / kLanes;
+  const ColliderArgs& ca;
+  V3 xpos;
+  float th;
+  uint32_t sub, group, shift;  // lane of the vertex, the vertex's lanes in the warp and their first
+  uint32_t win = 0, g = 0, node = 0;              // 4,096, 256 and 16 triangles being walked
+  uint32_t gmask = 0, nmask = 0, tmask = 0;       // their members still to visit
+  uint32_t stale = 0;                             // masks older than p: 1 tmask, 2 nmask, 4 gmask
+
+  // bit q of the result: test(base + q) for base + q < end
+  template <class F>
+  __device__ __forceinline__ uint32_t mask16(uint32_t base, uint32_t end, F&& test) const {
+    uint32_t out = 0;
+#pragma unroll
+    for (uint32_t e = 0; e < kEach; ++e) {
+      const uint32_t k = base + e * kLanes + sub;
+      const uint32_t b = __ballot_sync(group, k < end && test(k));
+      out |= ((b >> shift) & ((1u << kLanes) - 1u)) << (e * kLanes);
+    }
+    return out;
+  }
+  __device__ __forceinline__ uint32_t runs(uint32_t w, const SegBall& ball) const {
+    if (ball_far(ball, ca.cl4096[w], ca.cl4096[w].w + th)) return 0u;
+    return mask16(w * 16u, (ca.ntris + 255u) / 256u, [&](uint32_t k) {
+      const float4 c = ca.cl256[k];
+      return !ball_far(ball, c, c.w + th);
+    });
+  }
+  __device__ __forceinline__ uint32_t nodes(uint32_t r, const SegBall& ball) const {
+    return mask16(r * 16u, (ca.ntris + 15u) / 16u, [&](uint32_t k) {
+      const float4 c = ca.cl16[k];
+      return !ball_far(ball, c, c.w + th);
+    });
+  }
+  __device__ __forceinline__ uint32_t members(uint32_t r, const SegBall& ball, V3 p) const {
+    return mask16(r * 16u, ca.ntris, [&](uint32_t k) {
+      const float4 b = ca.bounds[k];
+      const float rr = b.w * 1.5f + th;
+      return !(ball_far(ball, b, rr) || seg_point_d2(xpos, p, mk(b)) > rr * rr);
+    });
+  }
+  // bits above the member k of its run of 16
+  static __device__ __forceinline__ uint32_t above(uint32_t k) { return 0xFFFEu << (k & 15u); }
+  // the next triangle to work at p, ca.ntris when there is none
+  __device__ __forceinline__ uint32_t next(const SegBall& ball, V3 p, uint32_t last) {
+    if (stale & 1u) tmask = members(node, ball, p) & above(last);
+    stale &= ~1u;
+    while (!tmask) {
+      if (stale & 2u) nmask = nodes(g, ball) & above(node);
+      stale &= ~2u;
+      while (!nmask) {
+        if (stale & 4u) gmask = runs(win, ball) & above(g);
+        stale &= ~4u;
+        while (!gmask) {
+          if (++win >= (ca.ntris + 4095u) / 4096u) {
+            win -= 1u;
+            return ca.ntris;
+          }
+          gmask = runs(win, ball);
+        }
+        g = win * 16u + uint32_t(__ffs(int(gmask)) - 1);
+        gmask &= gmask - 1u;
+        nmask = nodes(g, ball);
+      }
+      node = g * 16u + uint32_t(__ffs(int(nmask)) - 1);
+      nmask &= nmask - 1u;
+      tmask = members(node, ball, p);
+    }
+    const uint32_t t = node * 16u + uint32_t(__ffs(int(tmask)) - 1);
+    tmask &= tmask - 1u;
+    return t;
+  }
+};
+// Called by whole warps; kLanes consecutive lanes hold one vertex, live is the
+// same in all of them.
+template <uint32_t kLanes, class M>
+__device__ __forceinline__ void collide_vertex_lanes(bool live, uint32_t i, const M& m, const ColliderArgs& ca, float dt) {
+  const uint32_t lane = threadIdx.x & 31u;
+  float4 x = make_float4(0.f, 0.f, 0.f, 0.f), pr = x;
+  if (live) {
+    x = m.ldx(i);
+    live = x.w > 0.0f;
+  }
+  if (live) pr = m.ldp(i);
+  V3 p = mk(pr), xn = mk(x);
+  const V3 pinit = p, xpos = xn;
+  const float th = pr.w;
+  if (live) collide_prims(i, ca, dt, th, pinit, xn, p);
+  MeshState st;
+  st.bpos = p;
+  st.bn = mk(0.f, 0.f, 0.f);
+  const uint32_t shift = lane & ~(kLanes - 1u);
+  MeshWalk<kLanes> walk{ca, xpos, th, lane - shift, ((1u << kLanes) - 1u) << shift, shift};
+  SegBall ball = seg_ball(xpos, p);
+  uint32_t t = ca.ntris;
+  walk.win = 0xFFFFFFFFu;  // next() enters run 0
+  bool more = live;
+  while (true) {
+    if (more) {
+      t = walk.next(ball, p, t);
+      more = t < ca.ntris;
+    }
+    if (!__any_sync(0xffffffffu, more)) break;
+    if (more) {
+      const V3 before = p;
+      mesh_triangle(ca.tris[t], th, xpos, p, xn, dt, pinit, ca.recovery, st);
+      if (p.x != before.x || p.y != before.y || p.z != before.z) {
+        ball = seg_ball(xpos, p);
+        walk.stale = 7u;
+      }
+    }
+  }
+  if (!live) return;
+  if (!st.front && st.has_rec) contact(st.bpos, st.bn, st.bf, st.br, dt, pinit, xn, p);
+  if (walk.sub == 0u) {
+    m.stp(i, make_float4(p.x, p.y, p.z, pr.w));
+    m.stx(i, make_float4(xn.x, xn.y, xn.z, x.w));
+  }
+}
+template <uint32_t kLanes>
+__global__ void k_collision_lanes(uint32_t n, float4* __restrict__ x4, float4* __restrict__ p4, ColliderArgs ca,
+                                  float dt, const uint32_t* __restrict__ order) {
+  pdl_enter();
+  const uint32_t at = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
+  if (__all_sync(0xffffffffu, at >= n)) return;
+  const uint32_t i = at < n ? (order ? order[at] : at) : 0u;
+  collide_vertex_lanes<kLanes>(at < n, i, GMem<false>{x4, p4, nullptr}, ca, dt);
+}
+
 // ---------------------------------------------------------------------
 // persistent solver kernel
 // ---------------------------------------------------------------------
@@ -681,6 +826,7 @@ __device__ __forceinline__ bool grid_sync(GridBar* b, unsigned int expected, uns
 struct SolverArgs {
   uint32_t n, nsub, iters, npins, ndc, nbc;
   bool hascol, coupled, ddamp, bdamp, with_update;
+  bool iters_only;  // resident solver: the launch ends after the iterations of its one substep
   SubstepParams sp;
   float4 *x4, *p4, *v4;
   const uint2* dist_ids;

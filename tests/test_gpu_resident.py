@@ -6,6 +6,7 @@ stay on chip, and one that no longer fits."""
 import numpy as np
 import pytest
 
+from oracle import warmstart_ref as W
 from taremincloth_b200 import ClothSimulator, scenes
 
 pytestmark = pytest.mark.gpu
@@ -88,3 +89,24 @@ def test_mesh_without_triangles_and_single_step():
         s.set_pin(0, pos[0], 1.0)
         kernels = _both(s, 2, 4, 3)
         assert kernels[1] == 1
+
+
+@pytest.mark.parametrize("threshold", [None, float("inf"), 1e-4, -1.0])
+def test_chosen_persistent_solver_matches_the_default(threshold):
+    # without and with the warm start (never, as the residual says, always falling back)
+    out, stats = [], []
+    for mode in (1, 4):
+        s = _sheet(32, False, False)
+        s.set_launch_config(mode, 1)
+        s.set_solver_iterations(4)
+        if threshold is not None:
+            s.ws_set_params(W.random_params(np.random.default_rng(3), scale_head=0.05))
+            s.ws_enable(2, threshold)
+        for _ in range(2):
+            s.step(1.0 / 60.0, 6)
+        out.append([a.copy() for a in s.get_state()])
+        stats.append(s.ws_stats() if threshold is not None else None)
+    for a, b in zip(*out):
+        assert np.isfinite(b).all()
+        np.testing.assert_array_equal(a, b)
+    assert stats[0] == stats[1]
