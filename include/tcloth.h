@@ -544,6 +544,10 @@ tc_status tc_check_barrier_timeout(tc_sim *s, uint32_t spin_limit);
 tc_status tc_get_ccd_queue(tc_sim *s, uint32_t out[2]);
 /* Kernel launches in the recorded frame (kernel nodes of its CUDA graph). */
 tc_status tc_frame_kernel_count(tc_sim *s, uint32_t *count);
+/* Writes the recorded frame's launches and their dependencies as a DOT graph
+ * (cudaGraphDebugDotPrint), to look into what may overlap.  TC_ERR_INVALID
+ * before the first step after a change of settings. */
+tc_status tc_write_frame_graph(tc_sim *s, const char *path);
 /* Device time of the latest frame in milliseconds (CUDA events). */
 tc_status tc_last_frame_ms(tc_sim *s, float *ms);
 

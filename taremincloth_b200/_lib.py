@@ -124,6 +124,7 @@ SIGNATURES = {
     "tc_last_frame_ms": [_P, C.POINTER(_F)],
     "tc_set_profiling_enabled": [_P, _I],
     "tc_frame_kernel_count": [_P, C.POINTER(_U)],
+    "tc_write_frame_graph": [_P, C.c_char_p],
     "tc_set_persistent_solver": [_P, _I],
     "tc_set_launch_config": [_P, _I, _U],
     "tc_get_launch_limits": [_P, C.POINTER(_U), C.POINTER(_U)],

@@ -1551,19 +1551,19 @@ struct Sim {
     else if (ne < 50000u) launch_ee_v<4>(a, ss);
     else launch_ee_v<8>(a, ss);
   }
-  // normals: null, or the event after which they are there (recorded on another stream)
+  // normals: null, or the event after which they are there (recorded on another
+  // stream).  Every launch here may do contact work, which reads them: the
+  // filter too, on pairs that its list does not hold.
   void encode_ee(const SCArgs& a, cudaStream_t ss, cudaEvent_t normals = nullptr) {
     timed("sc_solve_ee", [&] {
       TC_CK(cudaMemsetAsync(ccd_n.p, 0, (1 + tcloth::kEeSeg) * sizeof(uint32_t), ss));
-      const bool listed = !ee_grouped && a.ee_cap;
-      if (normals && !listed) TC_CK(cudaStreamWaitEvent(ss, normals, 0));
+      if (normals) TC_CK(cudaStreamWaitEvent(ss, normals, 0));
       if (ee_grouped) {
         k_ee_grouped<<<grid(ne, 32 * tcloth::kEeWarps), 32 * tcloth::kEeWarps, 0, ss>>>(a);
       } else {
         if (a.ee_cap)
           launch_ee_cluster(a, ss);
         else k_ee<<<grid(ne, 8), 256, 0, ss>>>(a);
-        if (normals && listed) TC_CK(cudaStreamWaitEvent(ss, normals, 0));
         if (a.ee_cap) k_ee_pairs<<<tcloth::kEeSeg * tcloth::kEePairBlocks, 256, 0, ss>>>(a);
       }
     });
@@ -1629,8 +1629,8 @@ struct Sim {
     SCArgs a = sc_args();
     const bool edges_on = run_ee && ne > 0;
     const bool fork = edges_on && !profiling;
-    // star boxes and normals first: of the edge side only the contact work
-    // needs the normals
+    // star boxes and normals first: the edge side needs the normals once its
+    // hash is built
     auto stars = [&] {
       timed("sc_star_box", [&] {
         k_star_box<<<grid(n, 256), 256, 0, st>>>(n, star_off.p, star_idx.p, x4.p, p4.p, sbox.p, st_lo.p, st_hi.p,
@@ -2614,6 +2614,20 @@ struct Sim {
     return coupled || (auto_coupled && sdp > sm * 0.25f);
   }
 
+  cudaGraph_t capture_frame(float dt, uint32_t substeps, bool use_coupled) {
+    cudaGraph_t graph = nullptr;
+    TC_CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    try {
+      encode_frame(dt, substeps, use_coupled);
+    } catch (...) {
+      cudaStreamEndCapture(st, &graph);
+      if (graph) cudaGraphDestroy(graph);
+      throw;
+    }
+    TC_CK(cudaStreamEndCapture(st, &graph));
+    return graph;
+  }
+
   void launch_frame(float dt, uint32_t substeps) {
     if (n == 0) return;
     if (cluster_mode && can_cluster() && cl_stale) build_cluster_tables();  // before any capture
@@ -2635,16 +2649,7 @@ struct Sim {
     if (graph_dirty || !gexec || g_dt != dt || g_sub != substeps || g_coupled != use_coupled ||
         g_iters != run_iters()) {
       if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
-      cudaGraph_t graph = nullptr;
-      TC_CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      try {
-        encode_frame(dt, substeps, use_coupled);
-      } catch (...) {
-        cudaStreamEndCapture(st, &graph);
-        if (graph) cudaGraphDestroy(graph);
-        throw;
-      }
-      TC_CK(cudaStreamEndCapture(st, &graph));
+      cudaGraph_t graph = capture_frame(dt, substeps, use_coupled);
       size_t nn = 0;
       TC_CK(cudaGraphGetNodes(graph, nullptr, &nn));
       std::vector<cudaGraphNode_t> nodes(nn);
@@ -4035,6 +4040,19 @@ tc_status tc_check_barrier_timeout(tc_sim* s, uint32_t spin_limit) {
 
 tc_status tc_frame_kernel_count(tc_sim* s, uint32_t* count) {
   return guard([&] { Sim& m = S(s); need(count != nullptr, "count required"); *count = m.graph_kernels; });
+}
+
+tc_status tc_write_frame_graph(tc_sim* s, const char* path) {
+  return guard([&] {
+    Sim& m = S(s);
+    need(path != nullptr, "path required");
+    need(m.gexec != nullptr && !m.graph_dirty && !m.profiling && !m.ws_recording(),
+         "no frame is recorded for the present settings: step first");
+    cudaGraph_t graph = m.capture_frame(m.g_dt, m.g_sub, m.g_coupled);
+    const cudaError_t e = cudaGraphDebugDotPrint(graph, path, cudaGraphDebugDotFlagsKernelNodeParams);
+    cudaGraphDestroy(graph);
+    TC_CK(e);
+  });
 }
 
 tc_status tc_last_frame_ms(tc_sim* s, float* ms) {

@@ -985,6 +985,10 @@ class ClothSimulator:
         self._c(self._L.tc_frame_kernel_count(self._h, C.byref(v)))
         return v.value
 
+    def write_frame_graph(self, path):
+        """Write the recorded frame's launches and dependencies as a DOT graph."""
+        self._c(self._L.tc_write_frame_graph(self._h, str(path).encode()))
+
     def last_frame_ms(self):
         v = C.c_float()
         self._c(self._L.tc_last_frame_ms(self._h, C.byref(v)))
