@@ -1047,21 +1047,23 @@ struct Sim {
 
   // The state from host arrays (tc_set_positions_and_velocities) and back
   // (tc_get_state): the packed arrays cross the bus and are spread out on the
-  // device, through the star boxes' buffer, which only a self-collision pass
-  // uses and every pass fills anew.  Inverse masses go along when they may have
-  // changed.  (Building and reading padded arrays on the host took 3.8 ms of a
-  // 131,072-vertex frame.)
+  // device, each way through a buffer of its own that nothing else writes, so
+  // that a thread reading the state back gets a state whatever another thread
+  // launches between the kernel and the copies.  Inverse masses go along when
+  // they may have changed.  (Building and reading padded arrays on the host took
+  // 3.8 ms of a 131,072-vertex frame.)
+  DBuf<float> seek_buf, state_buf;  // 7 and 9 floats a vertex
   bool w_current = false;
   static constexpr uint32_t kSmallState = 16384;
-  std::vector<float> state_h;
   void seek(const float* pos, const float* vel) {
-    float* buf = reinterpret_cast<float*>(sbox.p);
+    float* buf = seek_buf.p;
     const size_t n3 = size_t(n) * 3;
+    std::unique_ptr<float[]> packed;
     if (n <= kSmallState && vel) {  // one copy: its latency is the cost
-      state_h.resize(3 * n3);
-      std::memcpy(state_h.data(), pos, n3 * sizeof(float));
-      std::memcpy(state_h.data() + n3, vel, n3 * sizeof(float));
-      TC_CK(cudaMemcpyAsync(buf, state_h.data(), 2 * n3 * sizeof(float), cudaMemcpyHostToDevice, st));
+      packed.reset(new float[2 * n3]);
+      std::memcpy(packed.get(), pos, n3 * sizeof(float));
+      std::memcpy(packed.get() + n3, vel, n3 * sizeof(float));
+      TC_CK(cudaMemcpyAsync(buf, packed.get(), 2 * n3 * sizeof(float), cudaMemcpyHostToDevice, st));
     } else {
       TC_CK(cudaMemcpyAsync(buf, pos, n3 * sizeof(float), cudaMemcpyHostToDevice, st));
       if (vel) TC_CK(cudaMemcpyAsync(buf + n3, vel, n3 * sizeof(float), cudaMemcpyHostToDevice, st));
@@ -1080,17 +1082,17 @@ struct Sim {
   }
   void get_state(float* x, float* p, float* v) {
     if (n == 0) return;
-    float* buf = reinterpret_cast<float*>(sbox.p);
-    k_state_out<<<grid(n, 256), 256, 0, st>>>(n, x4.p, p4.p, v4.p, buf);
+    const float* buf = state_buf.p;
+    k_state_out<<<grid(n, 256), 256, 0, st>>>(n, x4.p, p4.p, v4.p, state_buf.p);
     TC_CK(cudaGetLastError());
     const size_t n3 = size_t(n) * 3;
     float* out[3] = {x, p, v};
     if (n <= kSmallState) {
-      state_h.resize(3 * n3);
-      TC_CK(cudaMemcpyAsync(state_h.data(), buf, 3 * n3 * sizeof(float), cudaMemcpyDeviceToHost, st));
+      std::unique_ptr<float[]> packed(new float[3 * n3]);
+      TC_CK(cudaMemcpyAsync(packed.get(), buf, 3 * n3 * sizeof(float), cudaMemcpyDeviceToHost, st));
       TC_CK(cudaStreamSynchronize(st));
       for (int k = 0; k < 3; ++k)
-        if (out[k]) std::memcpy(out[k], state_h.data() + k * n3, n3 * sizeof(float));
+        if (out[k]) std::memcpy(out[k], packed.get() + k * n3, n3 * sizeof(float));
       return;
     }
     for (int k = 0; k < 3; ++k)
@@ -1253,6 +1255,7 @@ struct Sim {
     nrm.alloc(n);
     acc.alloc(size_t(n) * A_N);
     vcell.alloc(n); mlen.alloc(n); sbox.alloc(3 * size_t(n));
+    seek_buf.alloc(7 * size_t(n)); state_buf.alloc(9 * size_t(n));
     st_lo.alloc(m.star_idx.size() / 2); st_hi.alloc(m.star_idx.size() / 2); st_mz.alloc(m.star_idx.size() / 2);
     ecell.alloc(ne); eamin.alloc(ne); eamax.alloc(ne);
     ccd_q.alloc(size_t(ne) * 8 + 1024); ccd_n.alloc(1 + tcloth::kEeSeg);
