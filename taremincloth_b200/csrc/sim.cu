@@ -1058,7 +1058,10 @@ struct Sim {
   void seek(const float* pos, const float* vel) {
     float* buf = seek_buf.p;
     const size_t n3 = size_t(n) * 3;
+    // (copies from pageable memory may still read it after the call returns: both
+    // live until the stream has been waited for)
     std::unique_ptr<float[]> packed;
+    std::vector<float> w;
     if (n <= kSmallState && vel) {  // one copy: its latency is the cost
       packed.reset(new float[2 * n3]);
       std::memcpy(packed.get(), pos, n3 * sizeof(float));
@@ -1068,17 +1071,18 @@ struct Sim {
       TC_CK(cudaMemcpyAsync(buf, pos, n3 * sizeof(float), cudaMemcpyHostToDevice, st));
       if (vel) TC_CK(cudaMemcpyAsync(buf + n3, vel, n3 * sizeof(float), cudaMemcpyHostToDevice, st));
     }
-    if (!w_current) {
-      std::vector<float> w(orig_w);
+    const bool send_w = !w_current;
+    w_current = true;  // (a mass set by another thread from here on goes with the next seek)
+    if (send_w) {
+      w = orig_w;
       for (const auto& kv : pins) w[kv.first] = orig_w[kv.first] * (1.f - clamp_w(kv.second.weight));
       TC_CK(cudaMemcpyAsync(buf + 2 * n3, w.data(), size_t(n) * sizeof(float), cudaMemcpyHostToDevice, st));
     }
-    k_state_in<<<grid(n, 256), 256, 0, st>>>(n, buf, vel ? buf + n3 : nullptr, w_current ? nullptr : buf + 2 * n3,
+    k_state_in<<<grid(n, 256), 256, 0, st>>>(n, buf, vel ? buf + n3 : nullptr, send_w ? buf + 2 * n3 : nullptr,
                                               x4.p, p4.p, v4.p);
     TC_CK(cudaGetLastError());
     if (ws.ready) TC_CK(cudaMemsetAsync(ws.dprev.p, 0, size_t(n) * sizeof(float4), st));
     TC_CK(cudaStreamSynchronize(st));
-    w_current = true;
   }
   void get_state(float* x, float* p, float* v) {
     if (n == 0) return;
@@ -1179,9 +1183,10 @@ struct Sim {
     // work them in any order
     col_order_h = space_order(n, [&](uint32_t i, int k) { return m.pos[3 * size_t(i) + k]; });
     col_order.upload(col_order_h, st);
-    edge_order.upload(space_order(uint32_t(m.edges.size() / 2), [&](uint32_t e, int k) {
+    const std::vector<uint32_t> by_edge = space_order(uint32_t(m.edges.size() / 2), [&](uint32_t e, int k) {
       return 0.5f * (m.pos[3 * size_t(m.edges[2 * size_t(e)]) + k] + m.pos[3 * size_t(m.edges[2 * size_t(e) + 1]) + k]);
-    }), st);
+    });
+    edge_order.upload(by_edge, st);
     TC_CK(cudaStreamSynchronize(st));
     nd = uint32_t(m.dist.size());
     nb = uint32_t(m.bend.size());

@@ -52,3 +52,35 @@ def test_a_second_thread_reads_a_whole_state(n, busy):
         stop.set()
         t.join()
     assert not bad, (len(bad), bad[:3])
+
+
+@pytest.mark.parametrize("n", SIDES)
+def test_masses_follow_pins_and_settings_through_seeks(n):
+    """Inverse masses cross with the state only when they may have changed: a
+    simulator that was seeked before its pins and masses changed goes the same
+    way as one that had them from the start."""
+    sc = scenes.config2(n=n, subdiv=2)
+    rng = np.random.default_rng(3)
+    held = rng.choice(len(sc["positions"]), 6, replace=False)
+    v = rng.uniform(-0.1, 0.1, sc["positions"].shape).astype(np.float32)
+
+    def masses(s):
+        for k in held[:3]:
+            s.set_pin(int(k), sc["positions"][k], 1.0)
+        s.set_pin(int(held[3]), sc["positions"][held[3]], 0.5)
+        s.set_vertex_inv_masses(held[4:], np.array([0.0, 3.0], np.float32))
+
+    a, b = (scenes.build(ClothSimulator, sc) for _ in range(2))
+    masses(a)
+    b.set_positions_and_velocities(sc["positions"], v)
+    b.step(1.0 / 60.0, 4)
+    b.set_pin(int(held[5]), sc["positions"][held[5]], 1.0)
+    b.set_positions_and_velocities(sc["positions"], v)
+    b.release_pin(int(held[5]))
+    masses(b)
+    for _ in range(2):  # with the masses, then without
+        for s in (a, b):
+            s.set_positions_and_velocities(sc["positions"], v)
+            s.step(1.0 / 60.0, 4)
+        for x, y in zip(a.get_state(), b.get_state()):
+            np.testing.assert_array_equal(x, y)
