@@ -2200,8 +2200,9 @@ struct Sim {
   // The launch shape when the caller has not chosen one.  On chip where the
   // cloth fits one cluster: a colour step costs 0.5 to 1.1 us there.  A larger
   // single cloth runs one launch per colour, 2.1 us a step with programmatic
-  // launches.  The cooperative kernel's grid barrier costs 5.5 us a step, so
-  // it is left to batches (one launch per frame) and to callers that ask for it.
+  // launches.  The cooperative kernel's grid barrier costs 5.5 us a step, so it
+  // is left to batches that do not fit one cluster (one launch per frame) and to
+  // callers that ask for it.
   bool use_resident() const { return launch_auto && rs_ctas > 0; }
   bool use_persistent() const { return persistent && can_persist() && !(launch_auto && inst_vert_off.empty()); }
   // A mesh collider worth several lanes per vertex leaves the resident launch,
@@ -2211,8 +2212,18 @@ struct Sim {
   // self-collision, where the frame is one launch inside, 0.43 / 0.44, 0.59 /
   // 0.48, 0.76 / 0.52, 2.65 / 0.69.
   bool split_collision(bool use_coupled) const { return use_resident() && !use_coupled && collision_lanes() > 1u; }
+  // Coupled, such a collider runs once per iteration and cannot leave the
+  // launch: the frame then takes a launch per colour.  ms a frame of 10 x 5 over
+  // 1,280 / 20,480 triangles with the cloth on the body, resident, per colour
+  // and (for comparison) persistent: 288 vertices 6.4, 2.0, 10.1 / 19.1, 3.0,
+  // 22.6; 3,200: 4.2, 2.3, 9.5 / 14.8, 3.2, 25.9; 20,000: 8.4, 4.4, 8.5 / 28.9,
+  // 7.9, 22.6.  Before the cloth touches the two are level (3,200: 2.7, 2.1; 288:
+  // 1.7, 1.9).
+  bool resident_frame(bool use_coupled) const {
+    return use_resident() && !(use_coupled && collision_lanes() > 1u);
+  }
   void launch_solver(const SolverArgs& a) {
-    if (use_resident()) launch_resident(a);
+    if (resident_frame(a.coupled)) launch_resident(a);
     else launch_persistent(a);
   }
   // the persistent path is available: cooperative launch, and with bone
@@ -2527,7 +2538,8 @@ struct Sim {
       TC_CK(cudaGetLastError());
       return;
     }
-    if ((use_resident() || use_persistent()) && !profiling && !track_residual && !ws_recording()) {
+    const bool resident = resident_frame(use_coupled);
+    if ((resident || (use_persistent() && !use_resident())) && !profiling && !track_residual && !ws_recording()) {
       const SubstepParams sp = make_sp(dt / float(substeps));
       const bool split = split_collision(use_coupled);
       if (!self_collision && !edge_active() && !split) {
@@ -2548,7 +2560,7 @@ struct Sim {
           if (!sc || nsw) k_update_vel<<<grid(n, 256), 256, 0, st>>>(n, x4.p, p4.p, v4.p, sp.dt);
         }
       }
-      if (!use_resident()) TC_CK(cudaMemcpyAsync(h_err, &bar.p->err, sizeof(int), cudaMemcpyDeviceToHost, st));
+      if (!resident) TC_CK(cudaMemcpyAsync(h_err, &bar.p->err, sizeof(int), cudaMemcpyDeviceToHost, st));
       TC_CK(cudaGetLastError());
       return;
     }
