@@ -2205,13 +2205,13 @@ struct Sim {
   // callers that ask for it.
   bool use_resident() const { return launch_auto && rs_ctas > 0; }
   bool use_persistent() const { return persistent && can_persist() && !(launch_auto && inst_vert_off.empty()); }
-  // A mesh collider worth several lanes per vertex leaves the resident launch,
-  // whose 16 CTAs have a thread per vertex: ms a frame of 10 substeps inside /
+  // A mesh collider with a long walk leaves the resident launch, whose 16 CTAs
+  // have a thread per vertex: ms a frame of 10 substeps inside /
   // outside, 3,200 vertices with self-collision over 80 triangles 1.21 / 1.16,
   // 320: 1.36 / 1.20, 1,280: 1.52 / 1.22, 20,480: 3.38 / 1.41; without
   // self-collision, where the frame is one launch inside, 0.43 / 0.44, 0.59 /
   // 0.48, 0.76 / 0.52, 2.65 / 0.69.
-  bool split_collision(bool use_coupled) const { return use_resident() && !use_coupled && collision_lanes() > 1u; }
+  bool split_collision(bool use_coupled) const { return use_resident() && !use_coupled && long_walk(); }
   // Coupled, such a collider runs once per iteration and cannot leave the
   // launch: the frame then takes a launch per colour.  ms a frame of 10 x 5 over
   // 1,280 / 20,480 triangles with the cloth on the body, resident, per colour
@@ -2220,7 +2220,7 @@ struct Sim {
   // 7.9, 22.6.  Before the cloth touches the two are level (3,200: 2.7, 2.1; 288:
   // 1.7, 1.9).
   bool resident_frame(bool use_coupled) const {
-    return use_resident() && !(use_coupled && collision_lanes() > 1u);
+    return use_resident() && !(use_coupled && long_walk());
   }
   void launch_solver(const SolverArgs& a) {
     if (resident_frame(a.coupled)) launch_resident(a);
@@ -2496,19 +2496,25 @@ struct Sim {
   void launch_predict(const SubstepParams& sp) {
     launch_k(k_predict, grid(n, 256), 256, n, (const float4*)x4.p, p4.p, v4.p, sp, dlam.p, nd, blam.p, nb);
   }
+  // A mesh collider whose walk is worth more than a thread of a resident
+  // launch: below 256 triangles there is little to walk.
+  bool long_walk() const { return ntris >= 256u && n <= 32768u && !bone.enabled; }
   // Lanes per vertex of the mesh-collider pass.  A thread per vertex walks the
   // collider's spheres one after another, and up to 32,768 vertices are too few
   // warps to hide that: 16 lanes test a run at once up to 8,192 vertices, 8
-  // above.  More vertices fill the chip and the lanes' common work on each
-  // contact costs more than the shorter walk gives; below 256 triangles there
-  // is little to walk.  us per pass at 1 / 8 / 16 lanes, (vertices, triangles):
-  // (3,200, 1,280) 67 / 31 / 22, (3,200, 20,480) 302 / 63 / 42,
-  // (9,800, 5,120) 89 / 42 / 30, (29,282, 5,120) 84 / 49 / 45 and 93 / 87 / 94
-  // with the cloth on the body, (29,282, 320) 37 / 32 / 36, (29,282, 80) 21 /
-  // 31 / 35, (64,800, 20,480) 121 / 110 / 114 and 164 / 278 / 329 on the body,
-  // (131,072, 20,480) 105 / 182 / 219.
+  // above.  Above 20,480 vertices the lanes' common work on each contact weighs
+  // more than the walk of fewer than 4,096 triangles, and above 32,768 than any.
+  // us per pass at 1 / 8 / 16 lanes, (vertices, triangles): (3,200, 1,280) 67 /
+  // 31 / 22, (3,200, 20,480) 302 / 63 / 42, (9,800, 5,120) 89 / 42 / 30; at 1 / 8
+  // lanes with the cloth falling, touching the body and lying on it: (25,088,
+  // 320) 32 / 25, 36 / 36, 37 / 63, (25,088, 1,280) 37 / 25, 48 / 38, 53 / 81,
+  // (25,088, 5,120) 40 / 21, 89 / 52, 91 / 112, (25,088, 20,480) 36 / 18, 165 /
+  // 82, 172 / 159, (32,258, 1,280) 38 / 26, 46 / 48, 53 / 90, (32,258, 5,120)
+  // 39 / 22, 81 / 65, 87 / 127, (32,258, 20,480) 35 / 20, 154 / 93, 164 / 190;
+  // (64,800, 20,480) 121 / 110 falling and 164 / 278 on the body, (131,072,
+  // 20,480) 105 / 182.
   uint32_t collision_lanes() const {
-    if (ntris < 256u || n > 32768u || bone.enabled) return 1u;
+    if (!long_walk() || (n > 20480u && ntris < 4096u)) return 1u;
     return n <= 8192u ? 16u : 8u;
   }
   void launch_collision(const ColliderArgs& ca, float dts) {
