@@ -375,7 +375,7 @@ tc_status tc_set_hash_cell_size(tc_sim *s, float cell);
 tc_status tc_set_self_collision_variant(tc_sim *s, uint32_t ee_variant);
 /* Capacity, in (edge, edge) pairs, of the list through which variant 0
  * hands its counted pairs to the contact kernel (new; 0 = the default,
- * 24 per edge + 1024).  The list is split evenly among 256 segments; pairs
+ * 256 per edge up to 2^25, at least 24 per edge, + 1024).  The list is split evenly among 256 segments; pairs
  * past their segment's share are worked by the search kernel itself, so
  * results do not depend on it. */
 tc_status tc_set_ee_pair_list_capacity(tc_sim *s, uint64_t entries);
@@ -543,6 +543,10 @@ tc_status tc_check_barrier_timeout(tc_sim *s, uint32_t spin_limit);
  * the deferred edge-edge CCD kernel, and the queue capacity (pairs beyond it
  * run inline in the warp pass). */
 tc_status tc_get_ccd_queue(tc_sim *s, uint32_t out[2]);
+/* Diagnostics (new): out = edge pairs that the latest self-collision pass of
+ * variant 0 handed to the pair list, and how many of them did not fit (those
+ * were worked by the search kernel). */
+tc_status tc_get_ee_pair_list(tc_sim *s, uint64_t out[2]);
 /* Kernel launches in the recorded frame (kernel nodes of its CUDA graph). */
 tc_status tc_frame_kernel_count(tc_sim *s, uint32_t *count);
 /* Writes the recorded frame's launches and their dependencies as a DOT graph

@@ -1922,8 +1922,15 @@ __device__ __noinline__ void ee_list_ordered(const SCArgs& s, uint32_t ei, EeSea
 // more than max_search of them is searched again in the reference's order
 // (ee_list_ordered), as is every edge of a cluster whose pairs outgrow the
 // buffer.  The list's order is free.  A warp per edge (candidates over the
-// lanes) took 0.45 ms per pass on config 2 (391,682 edges, 13.6 counted pairs
+// lanes) took 0.45 ms per pass on config 2 (261,120 edges, 20 counted pairs
 // each), most of it bucket walks and searches.
+// The larger the buffer the fewer crowded edges are searched twice, but the
+// less L1 is left to the gathers.  us of this pass with 288 / 416 / 576 / 1,024
+// entries, layers of 58,080 edges pressed together to 4, 12, 20, 31 and 55 pairs
+// an edge (all of them listed but with 1,024): 59 / 60 / 62 / 79, 70 / 72 / 75 /
+// 98, 102 / 87 / 88 / 123, 206 / 140 / 123, 279 / 289 / 198.  A warp per edge
+// took 61, 68 and 73; the frame with it, 31 and 55 pairs an edge: 2.93 and 5.3
+// ms, 2.43 and 4.3 here.  More than 288 costs a frame of config 2 1 %.
 constexpr int kEeClusterWarps = 4;
 constexpr uint32_t kEePairBuf = 288;
 constexpr uint32_t kEeEdgeBits = 29;  // buffered pairs: edge of the cluster << 29 | candidate edge

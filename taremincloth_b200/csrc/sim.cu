@@ -1264,7 +1264,7 @@ struct Sim {
     st_lo.alloc(m.star_idx.size() / 2); st_hi.alloc(m.star_idx.size() / 2); st_mz.alloc(m.star_idx.size() / 2);
     ecell.alloc(ne); eamin.alloc(ne); eamax.alloc(ne);
     ccd_q.alloc(size_t(ne) * 8 + 1024); ccd_n.alloc(1 + tcloth::kEeSeg);
-    ee_q.alloc(size_t(ne) * 24 + 1024);
+    ee_q.alloc(ee_list_default(ne));
     vs_p.alloc(n); vs_q.alloc(n); vs_c.alloc(n); es_c.alloc(ne); es_v.alloc(ne); es_lo.alloc(ne); es_hi.alloc(ne);
     TC_CK(cudaMemsetAsync(acc.p, 0, size_t(n) * A_N * sizeof(int32_t), st));
     TC_CK(cudaMemsetAsync(nrm.p, 0, size_t(n) * sizeof(float4), st));
@@ -1496,7 +1496,15 @@ struct Sim {
   bool ee_grouped = false;
   // k_ee_cluster lists the counted pairs for k_ee_pairs (one lane per pair);
   // off: k_ee works them in the edge's warp; same pairs and results.  The list
-  // holds ee_list_entries pairs (0: all of ee_q, 24 per edge + 1024).
+  // holds ee_list_entries pairs (0: all of ee_q).
+  // Pairs past it are worked by the filter, which has half the warps of
+  // k_ee_pairs and is held up by its slowest block: with 24 an edge a cloth of
+  // 58,080 edges and 31 / 55 pairs an edge took 1.00 + 1.26 / 2.93 + 1.36 ms in
+  // the two, with room for all 0.21 + 1.49 / 0.28 + 2.97.  Room for the 256 that
+  // are counted at most by default, up to 268 MB of it; 24 an edge beyond.
+  static size_t ee_list_default(uint32_t edges) {
+    return std::max(size_t(edges) * 24, std::min(size_t(edges) * 256, size_t(1) << 25)) + 1024;
+  }
   bool ee_list = true;
   size_t ee_list_entries = 0;
   // narrow-phase pair record of the latest self-collision pass (off by default)
@@ -1547,8 +1555,8 @@ struct Sim {
   // times over, fewer below.  us per pass at 1 / 2 / 4 / 8 per warp, two layers
   // on a sphere: vertices 3,200: 21 / 23 / 32 / 45; 9,800: 53 / 51 / 46 / 70;
   // 29,282: 149 / 120 / 109 / 111; 131,072: 1258 / 1070 / 968 / 847.  Edges
-  // (with the pairs' contact math) 9,360: 30 / 28 / 31 / 36; 28,980: 54 / 47 /
-  // 46 / 48; 87,120: 125 / 99 / 84 / 78; 391,682: 940 / 733 / 572 / 532.
+  // (with the pairs' contact math) 6,240: 30 / 28 / 31 / 36; 19,320: 54 / 47 /
+  // 46 / 48; 58,080: 125 / 99 / 84 / 78; 261,120: 940 / 733 / 572 / 532.
   void launch_sc_solve(const SCArgs& a) {
     if (n < 5000u) launch_sc_v<1>(a);
     else if (n < 40000u) launch_sc_v<4>(a);
@@ -5116,6 +5124,24 @@ tc_status tc_get_ccd_queue(tc_sim* s, uint32_t out[2]) {
     }
     out[0] = q;
     out[1] = uint32_t(m.ccd_q.n);
+  });
+}
+
+tc_status tc_get_ee_pair_list(tc_sim* s, uint64_t out[2]) {
+  return guard([&] {
+    Sim& m = S(s);
+    need(out != nullptr, "out required");
+    uint32_t cnt[tcloth::kEeSeg] = {};
+    if (m.ccd_n.p) {
+      TC_CK(cudaMemcpyAsync(cnt, m.ccd_n.p + 1, sizeof cnt, cudaMemcpyDeviceToHost, m.st));
+      TC_CK(cudaStreamSynchronize(m.st));
+    }
+    const uint32_t cap = m.sc_args().ee_cap / tcloth::kEeSeg;
+    out[0] = out[1] = 0;
+    for (uint32_t c : cnt) {
+      out[0] += c;
+      out[1] += c > cap ? c - cap : 0u;
+    }
   });
 }
 

@@ -455,7 +455,7 @@ class ClothSimulator:
         self._c(self._L.tc_set_self_collision_variant(self._h, int(ee_variant)))
 
     def set_ee_pair_list_capacity(self, entries=0):
-        """Capacity of the E-E pair list of variant 0 (0 = 24 per edge + 1024);
+        """Capacity of the E-E pair list of variant 0 (0 = 256 per edge up to 2^25, at least 24 per edge);
         pairs past it are worked by the search kernel, with the same results."""
         self._c(self._L.tc_set_ee_pair_list_capacity(self._h, int(entries)))
 
@@ -998,6 +998,12 @@ class ClothSimulator:
         """(edge pairs deferred to the CCD kernel in the latest self-collision pass, capacity)"""
         out = np.zeros(2, _u32)
         self._c(self._L.tc_get_ccd_queue(self._h, _ptr(out)))
+        return int(out[0]), int(out[1])
+
+    def get_ee_pair_list(self):
+        """(edge pairs handed to the pair list in the latest self-collision pass, those that did not fit)"""
+        out = np.zeros(2, np.uint64)
+        self._c(self._L.tc_get_ee_pair_list(self._h, _ptr(out)))
         return int(out[0]), int(out[1])
 
     # ---- adaptive substeps and iterations (lib.rs:1788-1805, :1950-1965)
