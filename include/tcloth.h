@@ -517,8 +517,9 @@ tc_status tc_take_profile(tc_sim *s, char *names, size_t names_len, float *ms, u
  * separated by bounded grid barriers; off = one launch per colour.  Both give
  * the same bits.  Without a choice the library picks: the resident solver
  * (one thread-block cluster with the cloth or the batch on chip) where it fits
- * and no mesh collider of 256 triangles or more is coupled, else one launch per
- * colour; batched instances that do not fit run the persistent solver.  A
+ * and no mesh collider of 256 triangles or more (above 8,192 vertices: no 128
+ * simple colliders) is coupled, else one launch per colour; batched instances
+ * that do not fit run the persistent solver.  A
  * barrier that waits past its poll limit makes tc_step return TC_ERR_TIMEOUT.
  * New; the reference dispatches one pass per colour (dispatch.rs:1449-1455). */
 tc_status tc_set_persistent_solver(tc_sim *s, int enable);

@@ -2219,7 +2219,7 @@ struct Sim {
   // 320: 1.36 / 1.20, 1,280: 1.52 / 1.22, 20,480: 3.38 / 1.41; without
   // self-collision, where the frame is one launch inside, 0.43 / 0.44, 0.59 /
   // 0.48, 0.76 / 0.52, 2.65 / 0.69.
-  bool split_collision(bool use_coupled) const { return use_resident() && !use_coupled && long_walk(); }
+  bool split_collision(bool use_coupled) const { return use_resident() && !use_coupled && outgrows_resident(); }
   // Coupled, such a collider runs once per iteration and cannot leave the
   // launch: the frame then takes a launch per colour.  ms a frame of 10 x 5 over
   // 1,280 / 20,480 triangles with the cloth on the body, resident, per colour
@@ -2228,7 +2228,21 @@ struct Sim {
   // 7.9, 22.6.  Before the cloth touches the two are level (3,200: 2.7, 2.1; 288:
   // 1.7, 1.9).
   bool resident_frame(bool use_coupled) const {
-    return use_resident() && !(use_coupled && long_walk());
+    return use_resident() && !(use_coupled && outgrows_resident());
+  }
+  // The same goes for many simple colliders where a thread of the resident launch
+  // has more than one vertex: ms a frame of 10 x 4 inside / outside, 128 and 256
+  // spheres: 8,065 vertices (one each) 0.92 / 1.55, 1.23 / 1.88, coupled 1.9 /
+  // 2.6, 3.2 / 3.9; 10,225: 1.07 / 1.02, 1.54 / 1.34, coupled 2.5 / 2.6, 4.4 /
+  // 3.9; 19,013: 1.55 / 1.19, 2.49 / 1.50, coupled 4.1 / 2.7, 7.9 / 4.0 (6.2 with
+  // the persistent solver).
+  bool outgrows_resident() const { return long_walk() || (rs_chunk > tcloth::kResThreads && most_prims() >= 128u); }
+  // sphere, capsule and plane colliders that a vertex is tested against
+  uint32_t most_prims() const {
+    if (inst_prims_h.empty()) return uint32_t(prims_h.size());
+    uint32_t c = 0;
+    for (const auto& r : inst_prims_h) c = std::max(c, r.y);
+    return c;
   }
   void launch_solver(const SolverArgs& a) {
     if (resident_frame(a.coupled)) launch_resident(a);
