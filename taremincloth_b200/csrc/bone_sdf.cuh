@@ -26,6 +26,7 @@
 #pragma once
 #include <cuda_fp16.h>
 
+#include "morton.hpp"
 #include "vmath.cuh"
 
 namespace tcloth {
@@ -722,12 +723,8 @@ __global__ void k_mesh_codes(uint32_t n, const BakeTri* __restrict__ tris, MeshB
   uint32_t c = 0;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {  // (any order is exact; NaN goes to 0)
-    uint32_t v = uint32_t(fminf(fmaxf((u[a] - P.lmin[a]) / ext, 0.f), 1.f) * 1023.f);
-    v = (v * 0x00010001u) & 0xFF0000FFu;
-    v = (v * 0x00000101u) & 0x0F00F00Fu;
-    v = (v * 0x00000011u) & 0xC30C30C3u;
-    v = (v * 0x00000005u) & 0x49249249u;
-    c |= v << a;
+    const uint32_t v = uint32_t(fminf(fmaxf((u[a] - P.lmin[a]) / ext, 0.f), 1.f) * 1023.f);
+    c |= morton_spread10(v) << a;
   }
   code[t] = c;
   idx[t] = t;

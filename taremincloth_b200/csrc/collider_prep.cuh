@@ -9,6 +9,7 @@
 // are minima and maxima (exact in any order, NaN skipped the way the host's
 // std::fmin / std::min skip it), and the radix sort is stable.
 #pragma once
+#include "morton.hpp"
 #include "solver_kernels.cuh"
 
 namespace tcloth {
@@ -73,13 +74,6 @@ __global__ void __launch_bounds__(1024) k_col_bounds(uint32_t T, const MeshTri* 
     }
 }
 
-__device__ __forceinline__ uint32_t col_expand10(uint32_t v) {
-  v = (v * 0x00010001u) & 0xFF0000FFu;
-  v = (v * 0x00000101u) & 0x0F00F00Fu;
-  v = (v * 0x00000011u) & 0xC30C30C3u;
-  v = (v * 0x00000005u) & 0x49249249u;
-  return v;
-}
 __device__ __forceinline__ uint32_t col_quant(float f) {  // saturating float -> uint32
   if (!(f > 0.f)) return 0u;
   if (f >= 4294967295.f) return 0xFFFFFFFFu;
@@ -93,7 +87,7 @@ __global__ void k_col_codes(uint32_t T, const MeshTri* __restrict__ raw, const f
   uint32_t c[3];
   for (int a = 0; a < 3; ++a)
     c[a] = col_quant(fminf(fmaxf((col_cen(q, a) - box[a]) * box[3 + a], 0.f), 1.f) * 1023.f);
-  code[t] = (col_expand10(c[0]) << 2) | (col_expand10(c[1]) << 1) | col_expand10(c[2]);
+  code[t] = (morton_spread10(c[0]) << 2) | (morton_spread10(c[1]) << 1) | morton_spread10(c[2]);
   idx[t] = t;
 }
 

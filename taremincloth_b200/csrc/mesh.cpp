@@ -5,6 +5,7 @@
 // searches.  Insertion order is kept where the reference's output depends on
 // it (constraint order, strand neighbour order).
 #include "mesh.hpp"
+#include "morton.hpp"
 
 #include <algorithm>
 #include <cmath>
@@ -124,13 +125,6 @@ void bucket(const std::vector<uint32_t>& color, uint32_t ncol, std::vector<uint3
   for (size_t i = 0; i < color.size(); ++i) perm[f[color[i]]++] = uint32_t(i);
 }
 
-inline uint32_t expand10(uint32_t v) {
-  v = (v * 0x00010001u) & 0xFF0000FFu;
-  v = (v * 0x00000101u) & 0x0F00F00Fu;
-  v = (v * 0x00000011u) & 0xC30C30C3u;
-  v = (v * 0x00000005u) & 0x49249249u;
-  return v;
-}
 inline uint32_t sat_u32(float f) {
   if (!(f > 0.f)) return 0;
   if (f >= 4294967295.f) return UINT32_MAX;
@@ -150,7 +144,7 @@ uint32_t morton3(float px, float py, float pz, const float bmin[3], const float 
   uint32_t x = sat_u32(clamp01((px - bmin[0]) * inv[0]) * 1023.f);
   uint32_t y = sat_u32(clamp01((py - bmin[1]) * inv[1]) * 1023.f);
   uint32_t z = sat_u32(clamp01((pz - bmin[2]) * inv[2]) * 1023.f);
-  return (expand10(x) << 2) | (expand10(y) << 1) | expand10(z);
+  return (morton_spread10(x) << 2) | (morton_spread10(y) << 1) | morton_spread10(z);
 }
 
 // |(projection of p - e0 onto the edge e0->e1, distance from the edge line)|,
