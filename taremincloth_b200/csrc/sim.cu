@@ -82,9 +82,6 @@ __global__ void k_extract_positions(uint32_t n, const float4* __restrict__ x4, f
   out[3 * size_t(i) + 2] = x.z;
 }
 
-// Adaptive feedback (update_feedback_from_floats, dispatch.rs:356-429): the
-// largest per-axis displacement since the previous frame (max is order-free:
-// atomicMax on the bits of non-negative floats), then prev = x.
 // State from packed host layouts: pos, vel (or null: at rest) and w (or null:
 // the inverse masses on the device stand); thickness and layer stay.
 __global__ void k_state_in(uint32_t n, const float* __restrict__ pos, const float* __restrict__ vel,
@@ -113,6 +110,9 @@ __global__ void k_state_out(uint32_t n, const float4* __restrict__ x4, const flo
   }
 }
 
+// Adaptive feedback (update_feedback_from_floats, dispatch.rs:356-429): the
+// largest per-axis displacement since the previous frame (max is order-free:
+// atomicMax on the bits of non-negative floats), then prev = x.
 __global__ void k_fb_disp(uint32_t n, const float4* __restrict__ x4, float4* __restrict__ prev, float* out) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   float d = 0.f;
@@ -324,7 +324,7 @@ struct Mlp {
         k_mlp_layer_bwd_tc<<<bwd_grid_tc, 256, kWsBwdSmem, st>>>(
             MlpBwdTcArgs{n, x, dz.p, wb.p + wo, gw.p + wo, dx.p, adj_off, err});
       else
-        k_mlp_layer_bwd<<<gt, 128, 0, st>>>(MlpBwdArgs{n, 128, x, dz.p, wb.p + wo, gw.p + wo, dx.p, adj_off});
+        k_mlp_layer_bwd<<<gt, 128, 0, st>>>(MlpBwdArgs{n, x, dz.p, wb.p + wo, gw.p + wo, dx.p, adj_off});
     };
     auto below = [&](const float* z, uint32_t bo) {
       k_mlp_agg_act_bwd<<<row_grid, 32 * kWsRowWarps, 0, st>>>(n, dx.p, adj_off, adj_idx, z, dz.p, gw.p + bo);
@@ -2077,8 +2077,8 @@ struct Sim {
     for (uint32_t c : m.bend_cnt) rs_nsteps += c ? 1u : 0u;
     uint32_t k = 1;
     // about 512 vertices per CTA: one constraint per thread in a colour step.
-    // Fewer per CTA buys nothing (8,065 vertices: 0.89 ms a frame of 750 steps
-    // at 256 and 512, 0.97 at 1,024; 265 vertices: 0.20 on one CTA, 0.29 on two)
+    // (8,065 vertices, 750 steps a frame: 0.89 ms on 16 CTAs, 0.97 on 8; 265
+    // vertices: 0.20 ms on one CTA, 0.29 on two)
     while (k < tcloth::kResMaxCtas && (n + k - 1) / k > 512u) k *= 2;
     // constraints owned per CTA
     const uint32_t chunk = (n + k - 1) / k;

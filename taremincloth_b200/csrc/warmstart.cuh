@@ -415,16 +415,15 @@ __global__ void __launch_bounds__(32 * kWsRowWarps) k_mlp_agg_act_bwd(uint32_t n
   add_columns(d0, d1, sh, db);
 }
 
-// Weight gradient dW[kin][64] += X^T dZ over a 64-row tile (tensor cores),
-// and input gradient dX[n][kin] = dZ W^T.
+// Weight gradient dW[128][64] += X^T dZ over a 64-row tile (tensor cores),
+// and input gradient dX[n][128] = dZ W^T.
 struct MlpBwdArgs {
   uint32_t n;
-  int kin;
-  const __nv_bfloat16* x;    // [n][kin]
+  const __nv_bfloat16* x;    // [n][128]
   const __nv_bfloat16* dz;   // [n][64]
-  const __nv_bfloat16* w;    // [kin][64] (row-major weights = n-major for dZ W^T)
-  float* dw;                 // [kin][64]
-  float* dx;                 // [n][kin] or null; columns 64.. divided by the row's degree
+  const __nv_bfloat16* w;    // [128][64] (row-major weights = n-major for dZ W^T)
+  float* dw;                 // [128][64], added to
+  float* dx;                 // [n][128]; columns 64.. divided by the row's degree
   const uint32_t* adj_off;
 };
 __global__ void __launch_bounds__(128) k_mlp_layer_bwd(MlpBwdArgs a) {
@@ -433,7 +432,7 @@ __global__ void __launch_bounds__(128) k_mlp_layer_bwd(MlpBwdArgs a) {
   __shared__ __align__(16) __nv_bfloat16 wsm[128][kWsH + 8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t row0 = blockIdx.x * kWsRows;
-  const int kin = a.kin;
+  constexpr int kin = 2 * kWsH;
   for (int e = tid; e < kWsRows * kin; e += blockDim.x) {
     const int r = e / kin, c = e % kin;
     xs[r][c] = row0 + r < a.n ? a.x[size_t(row0 + r) * kin + c] : __float2bfloat16(0.f);
@@ -465,7 +464,6 @@ __global__ void __launch_bounds__(128) k_mlp_layer_bwd(MlpBwdArgs a) {
         atomicAdd(&a.dw[r * kWsH + c], acc[nt][q]);
       }
   }
-  if (!a.dx) return;
   // dX: M = 64 rows (16 per warp), N = kin, K = 64
   for (int nt = 0; nt < kin / 8; ++nt) {
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -555,7 +553,7 @@ struct MlpBwdTcArgs {
   const __nv_bfloat16* dz;  // [n][64]
   const __nv_bfloat16* w;   // [128][64] row-major weights
   float* dw;                // [128][64], added to
-  float* dx;                // [n][128] or null; columns 64.. divided by the row's degree
+  float* dx;                // [n][128]; columns 64.. divided by the row's degree
   const uint32_t* adj_off;
   int* err;
 };
@@ -631,7 +629,7 @@ __global__ void __launch_bounds__(256, 2) k_mlp_layer_bwd_tc(MlpBwdTcArgs a) {
     if (!ok) break;
     parity ^= 1u;
     tc_fence_after();
-    if (a.dx) {
+    {
       const uint32_t r = quad * 32 + lane, v = row0 + r;
 #pragma unroll
       for (int c0 = 0; c0 < 64; c0 += 32) {
