@@ -510,14 +510,18 @@ struct SegBall {
   V3 c;
   float h;
 };
-__device__ __forceinline__ SegBall seg_ball(V3 a, V3 b) {
+// (a vertex of negative thickness th: no end to the ball, since the groups'
+// spheres enclose their members' only for th >= 0, and the triangles' own test
+// is on r^2 whatever the sign)
+__device__ __forceinline__ SegBall seg_ball(V3 a, V3 b, float th) {
   const V3 c = (a + b) * 0.5f;
-  return SegBall{c, length(b - a) * 0.5005f + 1e-6f * (fabsf(c.x) + fabsf(c.y) + fabsf(c.z)) + 1e-6f};
+  const float h = length(b - a) * 0.5005f + 1e-6f * (fabsf(c.x) + fabsf(c.y) + fabsf(c.z)) + 1e-6f;
+  return SegBall{c, th < 0.f ? __int_as_float(0x7F800000) : h};
 }
-// true only when the segment is farther than r from the point
+// true only when the segment is farther than |r| from the point
 __device__ __forceinline__ bool ball_far(const SegBall& s, float4 g, float r) {
   const V3 d = s.c - mk(g);
-  const float R = r * 1.001f + s.h;
+  const float R = fabsf(r) * 1.001f + s.h;
   return dot(d, d) > R * R;
 }
 
@@ -586,7 +590,7 @@ __device__ __forceinline__ void collide_vertex_m(uint32_t i, const M& m, const C
     st.bpos = p;
     st.bn = mk(0.f, 0.f, 0.f);
     const uint32_t ng256 = (ca.ntris + 255u) / 256u, ng4096 = (ca.ntris + 4095u) / 4096u;
-    SegBall ball = seg_ball(xpos, p);
+    SegBall ball = seg_ball(xpos, p, th);
     for (uint32_t g4 = 0; g4 < ng4096; ++g4) {
       if (ball_far(ball, ca.cl4096[g4], ca.cl4096[g4].w + th)) continue;
       const uint32_t g_end = min((g4 + 1u) * 16u, ng256);
@@ -601,7 +605,7 @@ __device__ __forceinline__ void collide_vertex_m(uint32_t i, const M& m, const C
             const float r = b.w * 1.5f + th;
             if (ball_far(ball, b, r) || seg_point_d2(xpos, p, mk(b)) > r * r) continue;
             mesh_triangle(ca.tris[t], th, xpos, p, xn, dt, pinit, ca.recovery, st);
-            ball = seg_ball(xpos, p);  // a contact moves p
+            ball = seg_ball(xpos, p, th);  // a contact moves p
           }
         }
       }
@@ -744,7 +748,7 @@ __device__ __forceinline__ void collide_vertex_lanes(bool live, uint32_t i, cons
   st.bn = mk(0.f, 0.f, 0.f);
   const uint32_t shift = lane & ~(kLanes - 1u);
   MeshWalk<kLanes> walk{ca, xpos, th, lane - shift, ((1u << kLanes) - 1u) << shift, shift};
-  SegBall ball = seg_ball(xpos, p);
+  SegBall ball = seg_ball(xpos, p, th);
   uint32_t t = ca.ntris;
   walk.win = 0xFFFFFFFFu;  // next() enters run 0
   bool more = live;
@@ -758,7 +762,7 @@ __device__ __forceinline__ void collide_vertex_lanes(bool live, uint32_t i, cons
       const V3 before = p;
       mesh_triangle(ca.tris[t], th, xpos, p, xn, dt, pinit, ca.recovery, st);
       if (p.x != before.x || p.y != before.y || p.z != before.z) {
-        ball = seg_ball(xpos, p);
+        ball = seg_ball(xpos, p, th);
         walk.stale = 7u;
       }
     }
