@@ -641,8 +641,13 @@ __device__ __forceinline__ UnionBox union_box(const I3& cell, uint32_t todo, uin
   int32_t hy = __reduce_max_sync(0xffffffffu, in ? cell.y : INT32_MIN);
   int32_t hz = __reduce_max_sync(0xffffffffu, in ? cell.z : INT32_MIN);
   mine = in;
-  uint32_t ex = uint32_t(hx) - uint32_t(ox) + 3u, ey = uint32_t(hy) - uint32_t(oy) + 3u,
-           ez = uint32_t(hz) - uint32_t(oz) + 3u;
+  // (cells at both ends of the range, of positions that have run away: the
+  // difference + 3 would wrap to a small extent)
+  auto extent = [](int32_t lo, int32_t hi) {
+    const uint32_t d = uint32_t(hi) - uint32_t(lo);
+    return d <= kScCells ? d + 3u : kScCells + 1u;
+  };
+  uint32_t ex = extent(ox, hx), ey = extent(oy, hy), ez = extent(oz, hz);
   if (ex > kScCells || ey > kScCells || ez > kScCells || ex * ey * ez > kScCells) {
     const int lead = __ffs(todo) - 1;
     ox = hx = __shfl_sync(0xffffffffu, cell.x, lead);
@@ -656,8 +661,7 @@ __device__ __forceinline__ UnionBox union_box(const I3& cell, uint32_t todo, uin
       if (!((todo >> w) & 1u)) continue;
       const int32_t nx = min(ox, wx), ny = min(oy, wy), nz = min(oz, wz);
       const int32_t mx = max(hx, wx), my = max(hy, wy), mz = max(hz, wz);
-      const uint32_t fx = uint32_t(mx) - uint32_t(nx) + 3u, fy = uint32_t(my) - uint32_t(ny) + 3u,
-                     fz = uint32_t(mz) - uint32_t(nz) + 3u;
+      const uint32_t fx = extent(nx, mx), fy = extent(ny, my), fz = extent(nz, mz);
       if (fx > kScCells || fy > kScCells || fz > kScCells || fx * fy * fz > kScCells) continue;
       ox = nx; oy = ny; oz = nz;
       hx = mx; hy = my; hz = mz;
